@@ -14,6 +14,8 @@
 // 128-row query tile of one (batch, head) each), heaviest first under the causal
 // mask, dealt to the CTAs in boustrophedon order so the per-CTA totals even out.
 //
+// d_head 64 (prefill) splits O and the P V issue by softmax group, as described at SPLIT below;
+// the rest of this list is the general form.
 //   warps 8, 11        TMA producers (one lane each): Q per item and the K tiles / the V
 //   (one lane each)    tiles (128 keys) through mbarrier-guarded shared-memory rings,
 //                      128-byte swizzle.  K and V have a producer each so that K loads
@@ -48,7 +50,8 @@
 //                      cache the same warps first turn each V tile into the fp16 operand
 //                      of P V (the e4m3 prefill gets an fp16 V from a pre-pass instead).
 //
-// TMEM (all 512 columns): three score buffers [0,128) [128,256) [256,384), O [384,384+D).
+// TMEM (all 512 columns): three score buffers [0,128) [128,256) [256,384), O [384,384+D)
+// (SPLIT: two accumulators, [384,448) and [448,512)).
 #include <atomic>
 #include <cmath>
 
@@ -220,14 +223,24 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     using L = PrefillSmem<D, FP8, V8>;
     constexpr int NBOX = L::kNBox, NK = L::NK, NV = L::NV;
     constexpr uint32_t O_COL = kNU * 128;
+    // d_head 64 leaves TMEM for an accumulator of O per softmax group.  Each group then works on its
+    // key tiles with a running max of its own - no hand-over from tile to tile through shared memory,
+    // which cost ~340 clocks on every tile's critical path - and has a P V issuer of its own (warps 10
+    // and 11; one thread took ~830 clocks to issue a tile's 8 MMAs and commit, of ~1500 a tile);
+    // warp 8 loads V as well.  The epilogue merges the two (max, sum, O) of a row.  B200, f16:
+    // causal B*H=96 S=2048 91.0 -> 83.5 us, without a mask 149.7 -> 139.3 us, B*H=24 S=8192
+    // without a mask 548 -> 500 us (1500 -> 1300 clocks a tile).  d_head 128 has no TMEM for it, and
+    // grouped-query decode, bound by its cache reads, keeps the one accumulator.
+    constexpr bool SPLIT = (D == 64 && !GQA);
+    constexpr int NO = SPLIT ? 2 : 1;
     static_assert(NK <= kRing && NV <= kRing && kNU <= kRing, "a ring entry must not be reused before its waiters have looked");
-    static_assert(O_COL + D <= 512, "TMEM columns");
+    static_assert(O_COL + NO * D <= 512, "TMEM columns");
     constexpr uint32_t TMEM_COLS = 512;
     constexpr bool P_BF16 = BF16 && !FP8;                 // type of P (and of the V operand of P V)
     constexpr uint32_t FMT = P_BF16 ? kFmtBF16 : kFmtF16;
 
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bar_qf, bar_qe, bar_ofree, bar_odone;
+    __shared__ __align__(8) uint64_t bar_qf, bar_qe, bar_ofree[NO], bar_odone[NO];
     __shared__ __align__(8) uint64_t bar_kf[NK], bar_vf[NV];
     // completion rings of the two MMA streams: Q K^T / P V of tile g arrive on entry g % kRing
     __shared__ __align__(8) uint64_t bar_qk[kRing], bar_pvd[kRing];
@@ -256,8 +269,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (tid == 0) {
         mbar_init(smem_u32(&bar_qf), 1);
         mbar_init(smem_u32(&bar_qe), 1);
-        mbar_init(smem_u32(&bar_ofree), 4);              // the epilogue warps have read O
-        mbar_init(smem_u32(&bar_odone), 1);
+        for (int i = 0; i < NO; i++) {
+            mbar_init(smem_u32(&bar_ofree[i]), 4);       // the epilogue warps have read the accumulator
+            mbar_init(smem_u32(&bar_odone[i]), 1);
+        }
         for (int i = 0; i < NK; i++) mbar_init(smem_u32(&bar_kf[i]), 1);
         for (int i = 0; i < NV; i++) mbar_init(smem_u32(&bar_vf[i]), V8 ? 128 : 1);
         for (int i = 0; i < kRing; i++) { mbar_init(smem_u32(&bar_qk[i]), 1); mbar_init(smem_u32(&bar_pvd[i]), 1); }
@@ -353,12 +368,21 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             tma_load_3d(k_s + sk * L::kKBytes + b * L::kBox, &tm_k, smem_u32(&bar_kf[sk]),
                                         b * XSTEP, j * kBN, it.bh);
                     }
+                    if constexpr (SPLIT) {
+                        // V as well (warp 11 issues P V here): with four stages each the V slot, P V of tile
+                        // g - 4, frees before Q K^T may use the next K tile, which needs P V of tile g - 2
+                        const int sv = g % NV;
+                        if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
+                        mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), L::kVBytes);
+                        for (int b = 0; b < NBOX; b++)
+                            tma_load_3d(v_s + sv * L::kVBytes + b * L::kBox, &tm_v, smem_u32(&bar_vf[sv]), b * 64, j * kBN, it.bh);
+                    }
                 }
                 it_n++;
             }
         }
         __syncwarp();
-    } else if (warp == 11) {
+    } else if (!SPLIT && warp == 11) {
         // ------------------------------------------------------------ TMA producer: V
         if (lane == 0) {
             int g = 0, n_scrub = 0;
@@ -462,6 +486,47 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             it_n++;
         }
+    } else if (SPLIT && (warp == 10 || warp == 11)) {
+        // ------------------------------------------------------------ P V issuers, SPLIT
+        // Warp 10 the even tiles of the CTA's whole tile sequence into the first accumulator, warp 11 the
+        // odd ones into the second.
+        constexpr uint32_t idesc_pv = make_idesc(kBM, D, FMT, FMT, kMajorK, kMajorMN);
+        constexpr uint64_t hi_v = make_sdesc_hi(L::kBox, 1024);
+        const int par = warp - 10;
+        const uint32_t oc = tmem + O_COL + par * D;
+        int g0 = 0, used = 0;                             // items this accumulator has had
+        int u = par, u_phase = 0;                         // u == g % kNU, u_phase == (g / kNU) & 1
+        bool ok = true;
+        for (int r = 0; ok && r < n_rounds; r++) {
+            Item it;
+            if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
+            const int j0 = (g0 ^ par) & 1;
+            for (int j = j0; j < it.n_kv; j += 2) {
+                const int g = g0 + j;
+                const int sv = g % NV;
+                if (!mbar_wait(smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull)) { ok = false; break; }
+                if (!mbar_wait(smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull)) { ok = false; break; }
+                // the first P V of an item overwrites O: the epilogue of the last item must have read it
+                if (j == j0 && used > 0 && !mbar_wait(smem_u32(&bar_ofree[par]), (used - 1) & 1, ctl, kBarOFree)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t vb = v_s + sv * L::kVBytes;
+                const uint32_t pc = tmem + u * 128;         // P overwrote the first 64 columns of the tile's S
+#pragma unroll
+                for (int kk = 0; kk < kBN / 16; kk++) {
+                    const uint64_t db = make_sdesc(vb + kk * 2048, hi_v);
+                    if (lane == 0) mma_f16_ts(oc, pc + kk * 8, db, idesc_pv, (j > j0 || kk > 0) ? 1u : 0u);
+                }
+                if (lane == 0) {
+                    tc_commit(smem_u32(&bar_pvd[g % kRing]));               // score buffer and V slot are free
+                    if (j + 2 >= it.n_kv) tc_commit(smem_u32(&bar_odone[par]));   // the item's accumulator is complete
+                }
+                __syncwarp();
+                u += 2;
+                if (u >= kNU) { u -= kNU; u_phase ^= 1; }
+            }
+            if (j0 < it.n_kv) used++;
+            g0 += it.n_kv;
+        }
     } else if (warp == 10) {
         // ------------------------------------------------------------ P V issuer
         constexpr uint32_t idesc_pv = make_idesc(kBM, D, FMT, FMT, kMajorK, kMajorMN);
@@ -476,7 +541,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (!mbar_wait(smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull)) { ok = false; break; }
                 if (!mbar_wait(smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull)) { ok = false; break; }
                 // the first P V of an item overwrites O: the previous item's epilogue must have read it
-                if (j == 0 && it_n > 0 && !mbar_wait(smem_u32(&bar_ofree), (it_n - 1) & 1, ctl, kBarOFree)) { ok = false; break; }
+                if (j == 0 && it_n > 0 && !mbar_wait(smem_u32(&bar_ofree[0]), (it_n - 1) & 1, ctl, kBarOFree)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t vb = v_s + sv * L::kVBytes;
                 const uint32_t pc = tmem + u * 128;         // P overwrote the first 64 columns of the tile's S
@@ -487,7 +552,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 if (lane == 0) {
                     tc_commit(smem_u32(&bar_pvd[g % kRing]));               // score buffer and V slot are free
-                    if (j == it.n_kv - 1) tc_commit(smem_u32(&bar_odone));   // the item's O is complete
+                    if (j == it.n_kv - 1) tc_commit(smem_u32(&bar_odone[0]));   // the item's O is complete
                 }
                 __syncwarp();
                 if (u == kNU - 1) { u = 0; u_phase ^= 1; } else { u++; }
@@ -509,6 +574,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             return __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_epi), parity, ctl, kBarEpi));
         };
         int it_n = 0, g = 0;
+        uint32_t used = 0;                                // SPLIT: bit x: parity of the items accumulator x has had (g: first tile of the item)
         bool ok = true;
         for (int r = 0; ok && r < n_rounds; r++) {
             Item it;
@@ -568,10 +634,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // ---- epilogue of the item
             const int par = it_n & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats[par]), (it_n >> 1) & 1, ctl, kBarStats))) break;
-            const float m_a = xm[par][0][r_in_tile], m_b = xm[par][1][r_in_tile];
+            // a: the group that had the item's even tiles (SPLIT: so that the result does not depend on where
+            // in the CTA's tile sequence the item lies)
+            const int ga = SPLIT ? g & 1 : 0;
+            const float m_a = xm[par][ga][r_in_tile], m_b = xm[par][ga ^ 1][r_in_tile];
             const float m_fin = fmaxf(m_a, m_b);
-            const float l_run = xsum[par][0][r_in_tile] * ex2_approx(m_a - m_fin) +
-                                xsum[par][1][r_in_tile] * ex2_approx(m_b - m_fin);
+            const float l_run = xsum[par][ga][r_in_tile] * ex2_approx(m_a - m_fin) +
+                                xsum[par][ga ^ 1][r_in_tile] * ex2_approx(m_b - m_fin);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_stats_free[par]));
             float inv_l = 1.0f / l_run;
@@ -579,7 +648,60 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             const int row = it.q_start + r_in_tile;
             if (lse_out != nullptr && row < seq_len)
                 lse_out[static_cast<size_t>(it.bh) * seq_len + row] = kLn2 * (m_fin + log2f(l_run));
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_odone), it_n & 1, ctl, kBarODone))) break;
+            if constexpr (SPLIT) {
+                // an item of a single tile has used one accumulator only
+                const bool has_b = it.n_kv > 1;
+                g += it.n_kv;
+                bool w = mbar_wait(smem_u32(&bar_odone[ga]), (used >> ga) & 1, ctl, kBarODone);
+                if (has_b) w = w && mbar_wait(smem_u32(&bar_odone[ga ^ 1]), (used >> (ga ^ 1)) & 1, ctl, kBarODone);
+                used ^= has_b ? 3u : 1u << ga;
+                if (!__all_sync(0xffffffffu, w)) break;
+                tc_fence_after();
+                // the staging buffer must have been drained by the previous item's TMA store
+                if (tid == 384) tma_store_wait_read();
+                if (!rendezvous4(0)) break;
+                // O = (O_a 2^(m_a - m) + O_b 2^(m_b - m)) / l
+                const float f_a = ex2_approx(m_a - m_fin) * inv_l, f_b = ex2_approx(m_b - m_fin) * inv_l;
+#pragma unroll 1
+                for (int c = 0; c < D / 16; c++) {
+                    uint32_t oa[16], ob[16];
+                    tmem_ld16x2_wait(t_o + ga * D + c * 16, oa, t_o + (ga ^ 1) * D + c * 16, ob);
+                    if (c == D / 16 - 1) {                // out of TMEM: the next item may overwrite the accumulators
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(smem_u32(&bar_ofree[ga]));
+                            if (has_b) mbar_arrive(smem_u32(&bar_ofree[ga ^ 1]));
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {        // an accumulator the item has not used holds anything
+                        const float x = __uint_as_float(oa[i]) * f_a;
+                        oa[i] = __float_as_uint(has_b ? fmaf(__uint_as_float(ob[i]), f_b, x) : x);
+                    }
+#pragma unroll
+                    for (int g8 = 0; g8 < 2; g8++) {
+                        uint32_t w4[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            w4[e] = pack_16<BF16>(__uint_as_float(oa[g8 * 8 + 2 * e]), __uint_as_float(oa[g8 * 8 + 2 * e + 1]));
+                        const int c16 = c * 2 + g8;       // 8-element (16-byte) group index in the row
+                        const uint32_t addr = o_s + (c16 >> 3) * L::kBox + r_in_tile * 128 +
+                                              (((c16 & 7) ^ (r_in_tile & 7)) << 4);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w4[0]), "r"(w4[1]),
+                                     "r"(w4[2]), "r"(w4[3]) : "memory");
+                    }
+                }
+                fence_proxy_async_smem();
+                if (!rendezvous4(1)) break;
+                if (tid == 384) {
+                    for (int bx = 0; bx < NBOX; bx++) tma_store_3d(&tm_o, o_s + bx * L::kBox, bx * 64, it.q_start, it.bh);
+                    tma_store_commit();
+                }
+                it_n++;
+                continue;
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_odone[0]), it_n & 1, ctl, kBarODone))) break;
             tc_fence_after();
             if constexpr (GQA) {
                 // Result of this KV split for the rows that carry a (token, head) pair: with several
@@ -603,7 +725,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (c == D / 32 - 1) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bar_ofree));
+                        if (lane == 0) mbar_arrive(smem_u32(&bar_ofree[0]));
                     }
                     if (!seen) {                          // P was 2^(-inf + inf) there: not a number
 #pragma unroll
@@ -639,7 +761,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (c == D / 32 - 1) {                    // the whole row is out of TMEM: the next item may overwrite O
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bar_ofree));
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_ofree[0]));
                 }
 #pragma unroll
                 for (int g8 = 0; g8 < 4; g8++) {
@@ -672,7 +794,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int grp = warp >> 2;                        // group 0 owns even tiles (S0, P0), group 1 odd ones
         const int r_in_tile = (warp & 3) * 32 + lane;     // 0..127 == TMEM lane; one thread owns the whole row
         const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        const uint32_t t_o = tmem + lane_off + O_COL;
+        const uint32_t t_o = tmem + lane_off + O_COL + (SPLIT ? grp * D : 0);
         int g0 = 0, it_n = 0;
         bool ok = true;
 
@@ -735,10 +857,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const float tile_max = fmaxf(max3(a0, a1, a2), a3) * scale_log2;
                 // ---- the max in use: taken over from the previous tile (owned by the other group)
                 // unless this tile's max exceeds it by more than the threshold
+                // (SPLIT: from this thread's own previous tile; the groups' references are independent and
+                // meet in the epilogue)
                 float m_new = tile_max, m_prev_keep = tile_max;
                 bool changed = false;
                 const uint32_t slot = smem_u32(&m_slot[it_n & 1][r_in_tile]);
-                if (j > 0) {
+                if constexpr (SPLIT) {
+                    m_prev_keep = m_mine;
+                    if (j < 2) {
+                        m_new = fmaxf(tile_max, -1e30f);  // finite, so that a tile of -inf scores weighs nothing
+                    } else {
+                        changed = tile_max > m_mine + kRescaleThreshold;
+                        m_new = changed ? tile_max : m_mine;
+                    }
+                } else if (j > 0) {
                     // poll for the previous tile's entry (normally long there); bounded like every wait
                     uint32_t mb = 0, tag = 0;
                     const int w = bounded_wait(
@@ -760,8 +892,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     changed = tile_max > m_prev + kRescaleThreshold;
                     m_new = changed ? tile_max : m_prev;
                 }
-                asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(slot), "r"(__float_as_uint(m_new)),
-                             "r"(static_cast<uint32_t>(g)) : "memory");
+                if constexpr (!SPLIT)
+                    asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(slot), "r"(__float_as_uint(m_new)),
+                                 "r"(static_cast<uint32_t>(g)) : "memory");
                 if (m_new != m_mine) {                    // bring this thread's partial sum to the new reference
                     const float f = ex2_approx(m_mine - m_new);
                     lsum2 = fma2(lsum2, pack2(f, f), pack2(0.0f, 0.0f));
@@ -769,8 +902,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 
                 // ---- rare: the max in use grew -> rescale O in TMEM before this tile's P V
                 if (__any_sync(0xffffffffu, changed)) {
-                    // P V(g-1) must have finished accumulating into O
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, kBarPV))) { ok = false; break; }
+                    // the P V before this one must have finished accumulating into O
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - NO) % kRing]), ((g - NO) / kRing) & 1, ctl, kBarPV))) { ok = false; break; }
                     tc_fence_after();
                     // rows whose max did not change multiply by one; m_mine is not the previous max of
                     // the ROW (the other thread may have moved it), so the factor comes from m_prev

@@ -55,6 +55,7 @@
 #include <atomic>
 #include <cmath>
 
+#include "fast_div.h"
 #include "host_common.h"
 #include "ptx.cuh"
 #include "tmem_ld.cuh"
@@ -122,6 +123,9 @@ struct GqaDev {
     int tok_per_tile;       // tokens per query tile (row r of a tile: token r / group, head r % group)
     int n_qt;               // query tiles per (batch, KV head) = ceil(n_tok / tok_per_tile)
     int live_rows;          // rows of a tile a Q load writes = min(tok_per_tile, n_tok) * group
+    int heads_per_walk;     // (batch, KV head) pairs whose query tiles are walked together
+    // by n_splits; query tiles of a walk (prefill: of a group of heads); its heads; the last walk's heads; n_hkv
+    FastDiv by_splits, by_walk, by_heads, by_heads_last, by_hkv;
     const int* seq_lens;    // per-sequence KV lengths, or null: every sequence has seq_len keys
     const int* block_table; // paged cache: [batch][table_stride] page numbers, or null
     int table_stride;
@@ -131,14 +135,13 @@ struct GqaDev {
 // Work list: item index -> (query tile, head), heaviest first when causal.  In grouped-query
 // decode mode an item is (batch x KV head, query tile, KV split): key tiles [t0, t0 + n_kv) of that
 // head for the tokens from tok0 on.
-struct Item { int q_start, bh, n_kv, t0, split, kv_len, tok0; bool empty; };
+struct Item { int q_start, bh, n_kv, t0, split, kv_len, tok0, b, hkv; bool empty; };
 
 // Index of the partial result of tile row r: output row ((batch * n_tok + token) * Hq + query head),
 // then the KV split.
 __device__ __forceinline__ size_t gqa_partial_index(const GqaDev& gq, const Item& it, int r) {
-    const int b = it.bh / gq.n_hkv, hkv = it.bh - b * gq.n_hkv;
     const int tl = r / gq.group, g = r - tl * gq.group;
-    const size_t row = (static_cast<size_t>(b) * gq.n_tok + it.tok0 + tl) * (gq.n_hkv * gq.group) + hkv * gq.group + g;
+    const size_t row = (static_cast<size_t>(it.b) * gq.n_tok + it.tok0 + tl) * (gq.n_hkv * gq.group) + it.hkv * gq.group + g;
     return row * gq.n_splits + it.split;
 }
 
@@ -150,14 +153,21 @@ __device__ __forceinline__ bool get_item(int k, int n_items, int n_bh, int n_qti
         const int idx = k * G + c;                    // items are (nearly) equal: plain round-robin
         it.empty = false;
         if (idx >= n_items) return false;
-        const int bq = idx / gq.n_splits;             // (batch x KV head, query tile)
+        const int bq = gq.by_splits.quot(idx);        // (batch x KV head, query tile)
         it.split = idx - bq * gq.n_splits;
-        // the later query tiles see more keys: all heads' last tiles first
-        const int qt_rev = bq / n_bh;
-        it.bh = bq - qt_rev * n_bh;
+        // Heads are walked heads_per_walk at a time; within a walk the later query tiles, which see
+        // more keys, of all its heads come first (odd walks run light to heavy, as in the prefill below).
+        const int wi = gq.by_walk.quot(bq), rem = bq - wi * (gq.heads_per_walk * gq.n_qt);
+        const int h0 = wi * gq.heads_per_walk;
+        const bool last = h0 + gq.heads_per_walk > n_bh;
+        int qt_rev = (last ? gq.by_heads_last : gq.by_heads).quot(rem);
+        it.bh = h0 + rem - qt_rev * (last ? n_bh - h0 : gq.heads_per_walk);
+        if (wi & 1) qt_rev = gq.n_qt - 1 - qt_rev;
+        it.b = gq.by_hkv.quot(it.bh);
+        it.hkv = it.bh - it.b * gq.n_hkv;
         it.tok0 = (gq.n_qt - 1 - qt_rev) * gq.tok_per_tile;
         it.t0 = it.split * gq.tiles_per_split;
-        it.kv_len = gq.seq_lens ? min(seq_len, max(0, __ldg(gq.seq_lens + it.bh / gq.n_hkv))) : seq_len;
+        it.kv_len = gq.seq_lens ? min(seq_len, max(0, __ldg(gq.seq_lens + it.b))) : seq_len;
         // keys the tile's last token sees (the query tokens are the last n_tok entries of the cache)
         const int kv_vis = min(it.kv_len, it.kv_len - gq.n_tok + min(gq.n_tok, it.tok0 + gq.tok_per_tile));
         it.n_kv = min(gq.tiles_per_split, (max(kv_vis, 0) + kBN - 1) / kBN - it.t0);
@@ -180,19 +190,19 @@ __device__ __forceinline__ bool get_item(int k, int n_items, int n_bh, int n_qti
     // the extra index arithmetic (and the code it adds to every role) costs short work items 4-6 %.
     int qrank;
     if constexpr (GROUPED) {
-        const int per_group = gq.group * n_qtiles;
-        const int gi = idx / per_group, rem = idx - gi * per_group;
-        const int h0 = gi * gq.group, hin = min(gq.group, n_bh - h0);
-        qrank = rem / hin;
-        it.bh = h0 + rem - qrank * hin;
+        const int gi = gq.by_walk.quot(idx), rem = idx - gi * (gq.group * n_qtiles);
+        const int h0 = gi * gq.group;
+        const bool last = h0 + gq.group > n_bh;
+        qrank = (last ? gq.by_heads_last : gq.by_heads).quot(rem);
+        it.bh = h0 + rem - qrank * (last ? n_bh - h0 : gq.group);
         // Under the causal mask every group runs from its heaviest to its lightest tiles, a sawtooth
         // that the boustrophedon deal balances poorly (per-CTA totals up to 6 % above the mean on 32
         // heads of 64 tiles); odd groups run light to heavy instead, which halves that (a CTA's total
         // does not depend on the order in which it meets its items).
         if (CAUSAL && (gi & 1)) qrank = n_qtiles - 1 - qrank;
     } else {
-        qrank = idx / n_bh;
-        it.bh = idx % n_bh;
+        qrank = gq.by_heads.quot(idx);
+        it.bh = idx - qrank * n_bh;
     }
     const int qt = CAUSAL ? (n_qtiles - 1 - qrank) : qrank;
     it.q_start = qt * kBM;
@@ -314,7 +324,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     auto load_cache_tile = [&](uint32_t dst, const CUtensorMap* tm, uint32_t bar, const Item& it, int j) {
         constexpr int NB = FP8 ? 1 : NBOX;            // boxes per tile row: e4m3 rows are one 128-byte box
         constexpr int XS = FP8 ? 128 : 64;            // elements per box row
-        const int hkv = it.bh % gq.n_hkv, b = it.bh / gq.n_hkv;
+        const int hkv = it.hkv, b = it.b;
         const int r0 = (it.t0 + j) * kBN;
         if (gq.block_table == nullptr) {
             for (int bx = 0; bx < NB; bx++) tma_load_4d(dst + bx * L::kBox, tm, bar, bx * XS, r0, hkv, b);
@@ -349,8 +359,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     // the box holds only the live rows (token-major); the rest of the tile stays zero
                     mbar_arrive_expect_tx(smem_u32(&bar_qf), NLOAD * gq.live_rows * 128);
                     for (int b = 0; b < NLOAD; b++)
-                        tma_load_5d(q_s + b * L::kBox, &tm_q, smem_u32(&bar_qf), b * XSTEP, 0, it.tok0, it.bh % gq.n_hkv,
-                                    it.bh / gq.n_hkv);
+                        tma_load_5d(q_s + b * L::kBox, &tm_q, smem_u32(&bar_qf), b * XSTEP, 0, it.tok0, it.hkv, it.b);
                 } else {
                     mbar_arrive_expect_tx(smem_u32(&bar_qf), L::kQBytes);
                     for (int b = 0; b < NLOAD; b++)
@@ -703,14 +712,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_odone[0]), it_n & 1, ctl, kBarODone))) break;
             tc_fence_after();
+            bool seen = true;
             if constexpr (GQA) {
-                // Result of this KV split for the rows that carry a (token, head) pair: with several
-                // splits a normalised fp32 partial O and its LSE (the merge is a separate kernel), with
-                // one split the final 16-bit O and the LSE.
+                // Rows that carry a (token, head) pair.  With several KV splits each leaves a normalised fp32
+                // partial O and its LSE (the merge is a separate kernel).  With one split the 16-bit O of a
+                // tile with more than one warp of live rows goes the prefill's way below and only the LSE is
+                // written here: row-strided stores from registers hold O in TMEM, and with it the next item's
+                // P V, for the time of 128 x 16 scattered 16-byte writes (B=8 Hq=32 Hkv=8 T=Skv=2048 D=128:
+                // 441 us against 412).  Up to 32 live rows one warp's stores are the shorter way.
                 const bool live = r_in_tile < gq.live_rows && it.tok0 + r_in_tile / gq.group < gq.n_tok;
                 const size_t pidx = gqa_partial_index(gq, it, r_in_tile);
                 // a token with no visible key (a sequence shorter than the token count): O = 0, LSE = -inf
-                const bool seen = l_run > 0.0f;
+                seen = l_run > 0.0f;
                 if (!seen) inv_l = 0.0f;
                 const bool direct = gq.n_splits == 1;     // nothing to merge: this is the result
                 const float lse_val = seen ? kLn2 * (m_fin + log2f(l_run)) : -INFINITY;
@@ -718,38 +731,40 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!direct) gq.lse_part[pidx] = lse_val;
                     else if (gq.lse_final != nullptr) gq.lse_final[pidx] = lse_val;
                 }
+                if (!direct || gq.live_rows <= 32) {
 #pragma unroll 1
-                for (int c = 0; c < D / 32; c++) {
-                    uint32_t o[32];
-                    tmem_ld32_wait(t_o + c * 32, o);
-                    if (c == D / 32 - 1) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bar_ofree[0]));
-                    }
-                    if (!seen) {                          // P was 2^(-inf + inf) there: not a number
+                    for (int c = 0; c < D / 32; c++) {
+                        uint32_t o[32];
+                        tmem_ld32_wait(t_o + c * 32, o);
+                        if (c == D / 32 - 1) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(smem_u32(&bar_ofree[0]));
+                        }
+                        if (!seen) {                      // P was 2^(-inf + inf) there: not a number
 #pragma unroll
-                        for (int i = 0; i < 32; i++) o[i] = 0u;
-                    }
-                    if (live && direct) {
-                        uint4* dst = reinterpret_cast<uint4*>(gq.o_final + pidx * D + c * 32);
+                            for (int i = 0; i < 32; i++) o[i] = 0u;
+                        }
+                        if (live && direct) {
+                            uint4* dst = reinterpret_cast<uint4*>(gq.o_final + pidx * D + c * 32);
 #pragma unroll
-                        for (int e = 0; e < 4; e++)
-                            dst[e] = make_uint4(
-                                pack_16<BF16>(__uint_as_float(o[8 * e]) * inv_l, __uint_as_float(o[8 * e + 1]) * inv_l),
-                                pack_16<BF16>(__uint_as_float(o[8 * e + 2]) * inv_l, __uint_as_float(o[8 * e + 3]) * inv_l),
-                                pack_16<BF16>(__uint_as_float(o[8 * e + 4]) * inv_l, __uint_as_float(o[8 * e + 5]) * inv_l),
-                                pack_16<BF16>(__uint_as_float(o[8 * e + 6]) * inv_l, __uint_as_float(o[8 * e + 7]) * inv_l));
-                    } else if (live) {
-                        float4* dst = reinterpret_cast<float4*>(gq.o_part + pidx * D + c * 32);
+                            for (int e = 0; e < 4; e++)
+                                dst[e] = make_uint4(
+                                    pack_16<BF16>(__uint_as_float(o[8 * e]) * inv_l, __uint_as_float(o[8 * e + 1]) * inv_l),
+                                    pack_16<BF16>(__uint_as_float(o[8 * e + 2]) * inv_l, __uint_as_float(o[8 * e + 3]) * inv_l),
+                                    pack_16<BF16>(__uint_as_float(o[8 * e + 4]) * inv_l, __uint_as_float(o[8 * e + 5]) * inv_l),
+                                    pack_16<BF16>(__uint_as_float(o[8 * e + 6]) * inv_l, __uint_as_float(o[8 * e + 7]) * inv_l));
+                        } else if (live) {
+                            float4* dst = reinterpret_cast<float4*>(gq.o_part + pidx * D + c * 32);
 #pragma unroll
-                        for (int e = 0; e < 8; e++)
-                            dst[e] = make_float4(__uint_as_float(o[4 * e]) * inv_l, __uint_as_float(o[4 * e + 1]) * inv_l,
-                                                 __uint_as_float(o[4 * e + 2]) * inv_l, __uint_as_float(o[4 * e + 3]) * inv_l);
+                            for (int e = 0; e < 8; e++)
+                                dst[e] = make_float4(__uint_as_float(o[4 * e]) * inv_l, __uint_as_float(o[4 * e + 1]) * inv_l,
+                                                     __uint_as_float(o[4 * e + 2]) * inv_l, __uint_as_float(o[4 * e + 3]) * inv_l);
+                        }
                     }
+                    it_n++;
+                    continue;
                 }
-                it_n++;
-                continue;
             }
             // the staging buffer must have been drained by the previous item's TMA store
             if (tid == 384) tma_store_wait_read();
@@ -762,6 +777,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bar_ofree[0]));
+                }
+                if (GQA && !seen) {                       // P was 2^(-inf + inf) there: not a number
+#pragma unroll
+                    for (int i = 0; i < 32; i++) o[i] = 0u;
                 }
 #pragma unroll
                 for (int g8 = 0; g8 < 4; g8++) {
@@ -780,8 +799,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             fence_proxy_async_smem();
             if (!rendezvous4(1)) break;
             if (tid == 384) {
-                for (int bx = 0; bx < NBOX; bx++)
-                    tma_store_3d(&tm_o, o_s + bx * L::kBox, bx * 64, it.q_start, it.bh);
+                for (int bx = 0; bx < NBOX; bx++) {
+                    if constexpr (GQA)                    // the box holds the live rows, tokens past the last are clipped
+                        tma_store_5d(&tm_o, o_s + bx * L::kBox, bx * 64, 0, it.tok0, it.hkv, it.b);
+                    else
+                        tma_store_3d(&tm_o, o_s + bx * L::kBox, bx * 64, it.q_start, it.bh);
+                }
                 tma_store_commit();
             }
             it_n++;
@@ -1012,6 +1035,9 @@ int launch_instance(const fa_prefill_args& a, DeviceState* st, const CUtensorMap
     const int n_qtiles = (a.seq_len + kBM - 1) / kBM;
     const long long n_items = (long long)n_bh * n_qtiles;
     if (n_items > 0x7FFFFFFFll) return FA_ERR_INVALID_ARGUMENT;
+    order.by_walk = FastDiv((uint32_t)order.group * n_qtiles);
+    order.by_heads = FastDiv(order.group);
+    order.by_heads_last = FastDiv(n_bh % order.group ? n_bh % order.group : order.group);
     const unsigned grid = (unsigned)(n_items < st->sm_count ? n_items : st->sm_count);
     kernel<<<grid, kThreads, L::kTotal, static_cast<cudaStream_t>(a.stream)>>>(
         tq, tk, tv, to, a.lse, a.seq_len, n_bh, n_qtiles, (int)n_items, a.scale * kLog2e, a.q_scale,
@@ -1022,7 +1048,7 @@ int launch_instance(const fa_prefill_args& a, DeviceState* st, const CUtensorMap
 
 template <int D, bool BF16, bool FP8>
 int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& tq, const CUtensorMap& tk,
-                        const CUtensorMap& tv) {
+                        const CUtensorMap& tv, const CUtensorMap& to) {
     using L = PrefillSmem<D, FP8>;
     auto kernel = prefill_kernel<D, false, BF16, FP8, true, false>;
     static bool configured[64] = {};
@@ -1038,11 +1064,18 @@ int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& 
     const unsigned grid = (unsigned)(n_items < st->sm_count ? n_items : st->sm_count);
     int page_shift = 0;
     while ((1 << page_shift) < g.page_size) page_shift++;
+    // With several query tiles a head's K and V are read once per tile: walked over all heads at once
+    // they only come from L2 while the whole cache fits there.  B=8 Hkv=8 Skv=4096 D=128, 512 new tokens
+    // (134 MB of cache, 16 query tiles): 301 us over all heads, 269 us 8 heads at a time.  A single query
+    // tile reads everything once, in any order.
+    const int walk = n_qt > 1 ? heads_per_group(n_bh, g.kv_len, g.d_head, FP8 ? 1 : 2) : n_bh;
+    const int last_heads = n_bh % walk ? n_bh % walk : walk;
     const GqaDev gq{g.o_part, g.lse_part, static_cast<uint16_t*>(g.o_final), g.lse_final, g.n_splits,
                     g.tiles_per_split, g.group, g.n_kv_heads,
-                    g.n_tok, tok_per_tile, n_qt, tok_per_tile * g.group, g.seq_lens, g.block_table, g.table_stride,
+                    g.n_tok, tok_per_tile, n_qt, tok_per_tile * g.group, walk,
+                    FastDiv(g.n_splits), FastDiv((uint32_t)walk * n_qt), FastDiv(walk), FastDiv(last_heads), FastDiv(g.n_kv_heads), g.seq_lens, g.block_table, g.table_stride,
                     page_shift};
-    kernel<<<grid, kThreads, L::kTotal, g.stream>>>(tq, tk, tv, tq, nullptr, g.kv_len, n_bh, 1, (int)n_items,
+    kernel<<<grid, kThreads, L::kTotal, g.stream>>>(tq, tk, tv, to, nullptr, g.kv_len, n_bh, 1, (int)n_items,
                                                     g.scale * kLog2e, g.q_scale, g.k_scale, g.v_scale, st->status, gq);
     FA_CUDA_TRY(cudaGetLastError());
     return FA_OK;
@@ -1088,13 +1121,16 @@ int launch_prefill_16bit(const fa_prefill_args& a, DeviceState* st, int variant)
 }
 
 int launch_decode_gqa(const GqaLaunch& g, DeviceState* st) {
-    CUtensorMap tq, tk, tv;
+    CUtensorMap tq, tk, tv, to;
     int rc;
     // Q [B, T, Hq, D]: one box per (batch, KV head) with its group x T rows, token-major
     const bool e4m3 = g.dtype == FA_DTYPE_E4M3;
     const uint32_t box_cols = e4m3 ? 128 : 64;           // 128 bytes of a row either way
     if ((rc = make_tensor_map_q5(&tq, g.q, g.dtype, g.d_head, g.group, g.n_tok, g.n_kv_heads, g.batch, box_cols)) != FA_OK)
         return rc;
+    // O has Q's shape: with one KV split the epilogue stores its tiles through this map
+    if ((rc = make_tensor_map_q5(&to, g.o_final, e4m3 ? FA_DTYPE_BF16 : g.dtype, g.d_head, g.group, g.n_tok, g.n_kv_heads,
+                                 g.batch, 64)) != FA_OK) return rc;
     // dense / strided cache: (d, key, KV head, batch); paged: (d, key in page, KV head, page)
     const bool paged = g.block_table != nullptr;
     const uint64_t rows = paged ? (uint64_t)g.page_size : (uint64_t)g.kv_len;
@@ -1105,11 +1141,11 @@ int launch_decode_gqa(const GqaLaunch& g, DeviceState* st) {
                                  g.head_stride, bstride, box_cols, box_rows)) != FA_OK) return rc;
     if ((rc = make_tensor_map_4d(&tv, g.v, g.dtype, g.d_head, rows, g.n_kv_heads, blocks, g.row_stride,
                                  g.head_stride, bstride, box_cols, box_rows)) != FA_OK) return rc;
-    if (e4m3) return launch_gqa_instance<128, true, true>(g, st, tq, tk, tv);
+    if (e4m3) return launch_gqa_instance<128, true, true>(g, st, tq, tk, tv, to);
     const bool bf = g.dtype == FA_DTYPE_BF16;
     if (g.d_head == 64)
-        return bf ? launch_gqa_instance<64, true, false>(g, st, tq, tk, tv) : launch_gqa_instance<64, false, false>(g, st, tq, tk, tv);
-    return bf ? launch_gqa_instance<128, true, false>(g, st, tq, tk, tv) : launch_gqa_instance<128, false, false>(g, st, tq, tk, tv);
+        return bf ? launch_gqa_instance<64, true, false>(g, st, tq, tk, tv, to) : launch_gqa_instance<64, false, false>(g, st, tq, tk, tv, to);
+    return bf ? launch_gqa_instance<128, true, false>(g, st, tq, tk, tv, to) : launch_gqa_instance<128, false, false>(g, st, tq, tk, tv, to);
 }
 
 

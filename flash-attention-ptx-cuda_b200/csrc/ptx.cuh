@@ -33,6 +33,16 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
     return t;
 }
 
+// True in one lane of a converged warp, always the same one.  An issuing warp walks its loop as a whole and
+// guards its tcgen05 / TMA instructions with this: unlike after `lane == 0` the compiler then knows that a
+// single lane is active and that addresses and descriptors are warp-uniform, and issues them without moving
+// every operand to a uniform register under a divergence check.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------

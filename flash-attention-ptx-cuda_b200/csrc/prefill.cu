@@ -347,15 +347,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // ------------------------------------------------------------ TMA producer: Q and K
         // (K and V have a producer each: a K slot frees when its Q K^T is done, a V slot only when
         // its P V is done, much later; one in-order producer would hold K loads back behind V.)
-        if (lane == 0) {
-            constexpr int NLOAD = FP8 ? 1 : NBOX;         // boxes per Q / K tile
-            constexpr int XSTEP = FP8 ? 128 : 64;         // elements per box row
-            int g = 0, it_n = 0;
-            bool ok = true;
-            for (int r = 0; ok && r < n_rounds; r++) {
-                Item it;
-                if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
-                if (it_n > 0 && !mbar_wait(smem_u32(&bar_qe), (it_n - 1) & 1, ctl, kBarQEmpty)) break;
+        // An elected lane of the whole warp issues here too: a paged cache of 16-key pages takes 32 loads
+        // a key tile (B=16 Hkv=8 Skv<=4096 D=128 56.7 -> 43.9 us; a [B, S, H, D] cache 38.5 -> 36.2).
+        constexpr int NLOAD = FP8 ? 1 : NBOX;             // boxes per Q / K tile
+        constexpr int XSTEP = FP8 ? 128 : 64;             // elements per box row
+        int g = 0, it_n = 0;
+        bool ok = true;
+        for (int r = 0; ok && r < n_rounds; r++) {
+            Item it;
+            if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
+            if (it_n > 0 && !mbar_wait(smem_u32(&bar_qe), (it_n - 1) & 1, ctl, kBarQEmpty)) break;
+            if (elect_one()) {
                 if constexpr (GQA) {
                     // the box holds only the live rows (token-major); the rest of the tile stays zero
                     mbar_arrive_expect_tx(smem_u32(&bar_qf), NLOAD * gq.live_rows * 128);
@@ -366,10 +368,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     for (int b = 0; b < NLOAD; b++)
                         tma_load_3d(q_s + b * L::kBox, &tm_q, smem_u32(&bar_qf), b * XSTEP, it.q_start, it.bh);
                 }
-                for (int j = 0; j < it.n_kv; j++, g++) {
-                    const int sk = g % NK;
-                    // the slot was last read by Q K^T of tile g - NK
-                    if (g >= NK && !mbar_wait(smem_u32(&bar_qk[(g - NK) % kRing]), ((g - NK) / kRing) & 1, ctl, kBarKEmpty)) { ok = false; break; }
+            }
+            __syncwarp();
+            for (int j = 0; j < it.n_kv; j++, g++) {
+                const int sk = g % NK;
+                // the slot was last read by Q K^T of tile g - NK
+                if (g >= NK && !mbar_wait(smem_u32(&bar_qk[(g - NK) % kRing]), ((g - NK) / kRing) & 1, ctl, kBarKEmpty)) { ok = false; break; }
+                if (elect_one()) {
                     mbar_arrive_expect_tx(smem_u32(&bar_kf[sk]), L::kKBytes);
                     if constexpr (GQA) {
                         load_cache_tile(k_s + sk * L::kKBytes, &tm_k, smem_u32(&bar_kf[sk]), it, j);
@@ -378,78 +383,81 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             tma_load_3d(k_s + sk * L::kKBytes + b * L::kBox, &tm_k, smem_u32(&bar_kf[sk]),
                                         b * XSTEP, j * kBN, it.bh);
                     }
-                    if constexpr (SPLIT) {
-                        // V as well (warp 11 issues P V here): with four stages each the V slot, P V of tile
-                        // g - 4, frees before Q K^T may use the next K tile, which needs P V of tile g - 2
-                        const int sv = g % NV;
-                        if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
+                }
+                __syncwarp();
+                if constexpr (SPLIT) {
+                    // V as well (warp 11 issues P V here): with four stages each the V slot, P V of tile
+                    // g - 4, frees before Q K^T may use the next K tile, which needs P V of tile g - 2
+                    const int sv = g % NV;
+                    if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
+                    if (elect_one()) {
                         mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), L::kVBytes);
                         for (int b = 0; b < NBOX; b++)
                             tma_load_3d(v_s + sv * L::kVBytes + b * L::kBox, &tm_v, smem_u32(&bar_vf[sv]), b * 64, j * kBN, it.bh);
                     }
+                    __syncwarp();
                 }
-                it_n++;
             }
+            it_n++;
         }
-        __syncwarp();
     } else if (!SPLIT && warp == 11) {
         // ------------------------------------------------------------ TMA producer: V
-        if (lane == 0) {
-            int g = 0, n_scrub = 0;
-            bool ok = true;
-            for (int r = 0; ok && r < n_rounds; r++) {
-                Item it;
-                if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
-                for (int j = 0; j < it.n_kv; j++, g++) {
-                    if constexpr (V8) {
-                        // e4m3 V lands in its own buffers; warps 12-15 turn it into the fp16 operand.
-                        const int s8 = g & 1;
-                        if (g >= 2 && !mbar_wait(smem_u32(&bar_v8e[s8]), ((g >> 1) - 1) & 1, ctl, kBarV8Empty)) { ok = false; break; }
+        int g = 0, n_scrub = 0;
+        bool ok = true;
+        for (int r = 0; ok && r < n_rounds; r++) {
+            Item it;
+            if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
+            for (int j = 0; j < it.n_kv; j++, g++) {
+                if constexpr (V8) {
+                    // e4m3 V lands in its own buffers; warps 12-15 turn it into the fp16 operand.
+                    const int s8 = g & 1;
+                    if (g >= 2 && !mbar_wait(smem_u32(&bar_v8e[s8]), ((g >> 1) - 1) & 1, ctl, kBarV8Empty)) { ok = false; break; }
+                    if (elect_one()) {
                         mbar_arrive_expect_tx(smem_u32(&bar_v8f[s8]), L::kV8Bytes);
-                        if constexpr (GQA)
-                            load_cache_tile(v8_s + s8 * L::kV8Bytes, &tm_v, smem_u32(&bar_v8f[s8]), it, j);
-                        else
-                            tma_load_3d(v8_s + s8 * L::kV8Bytes, &tm_v, smem_u32(&bar_v8f[s8]), 0, j * kBN, it.bh);
+                        load_cache_tile(v8_s + s8 * L::kV8Bytes, &tm_v, smem_u32(&bar_v8f[s8]), it, j);
+                    }
+                    __syncwarp();
+                } else {
+                    const int sv = g % NV;
+                    // the slot was last read by P V of tile g - NV
+                    if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
+                    const uint32_t vdst = v_s + sv * L::kVBytes;
+                    if constexpr (GQA) {
+                        // Rows of the sequence's last tile past its end are stale cache contents when the
+                        // cache is paged or longer than the sequence (a dense cache reads them as zero).
+                        // P is exactly 0 there, but 0 x NaN would still poison O, so those rows of V are
+                        // cleared before the P V issuer may see the tile: the load completes on a private
+                        // barrier, this warp clears the rows and then releases the tile itself.
+                        const int valid = it.kv_len - (it.t0 + j) * kBN;      // rows of this tile inside the sequence
+                        const bool scrub = valid < kBN && (gq.seq_lens != nullptr || gq.block_table != nullptr);
+                        const uint32_t full = scrub ? smem_u32(&bar_vraw) : smem_u32(&bar_vf[sv]);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(full, L::kVBytes);
+                            load_cache_tile(vdst, &tm_v, full, it, j);
+                        }
+                        __syncwarp();
+                        if (scrub) {
+                            if (!mbar_wait(full, n_scrub & 1, ctl, kBarVFull)) { ok = false; break; }
+                            n_scrub++;
+                            for (int i = lane; i < (kBN - valid) * NBOX * 8; i += 32)     // 16 bytes each
+                                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(
+                                    vdst + (i >> 3) % NBOX * L::kBox + (valid + (i >> 3) / NBOX) * 128 + (i & 7) * 16), "r"(0u) : "memory");
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (elect_one()) mbar_arrive(smem_u32(&bar_vf[sv]));
+                            __syncwarp();
+                        }
                     } else {
-                        const int sv = g % NV;
-                        // the slot was last read by P V of tile g - NV
-                        if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
-                        if constexpr (GQA) {
-                            // Rows of the sequence's last tile past its end are stale cache contents when the
-                            // cache is paged or longer than the sequence (a dense cache reads them as zero).
-                            // P is exactly 0 there, but 0 x NaN would still poison O, so those rows of V are
-                            // cleared before the P V issuer may see the tile: the load completes on a private
-                            // barrier, this thread clears the rows and then releases the tile itself.
-                            const int valid = it.kv_len - (it.t0 + j) * kBN;      // rows of this tile inside the sequence
-                            const bool scrub = valid < kBN && (gq.seq_lens != nullptr || gq.block_table != nullptr);
-                            const uint32_t vdst = v_s + sv * L::kVBytes;
-                            if (!scrub) {
-                                mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), L::kVBytes);
-                                load_cache_tile(vdst, &tm_v, smem_u32(&bar_vf[sv]), it, j);
-                            } else {
-                                mbar_arrive_expect_tx(smem_u32(&bar_vraw), L::kVBytes);
-                                load_cache_tile(vdst, &tm_v, smem_u32(&bar_vraw), it, j);
-                                if (!mbar_wait(smem_u32(&bar_vraw), n_scrub & 1, ctl, kBarVFull)) { ok = false; break; }
-                                n_scrub++;
-                                for (int row = valid; row < kBN; row++)
-                                    for (int b = 0; b < NBOX; b++)
-                                        for (int q16 = 0; q16 < 8; q16++)
-                                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(
-                                                vdst + b * L::kBox + row * 128 + q16 * 16), "r"(0u) : "memory");
-                                fence_proxy_async_smem();
-                                mbar_arrive(smem_u32(&bar_vf[sv]));
-                            }
-                        } else {
+                        if (elect_one()) {
                             mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), L::kVBytes);
                             for (int b = 0; b < NBOX; b++)
-                                tma_load_3d(v_s + sv * L::kVBytes + b * L::kBox, &tm_v, smem_u32(&bar_vf[sv]),
-                                            b * 64, j * kBN, it.bh);
+                                tma_load_3d(vdst + b * L::kBox, &tm_v, smem_u32(&bar_vf[sv]), b * 64, j * kBN, it.bh);
                         }
+                        __syncwarp();
                     }
                 }
             }
         }
-        __syncwarp();
     } else if (warp == 9) {
         // ------------------------------------------------------------ Q K^T issuer
         // The whole warp walks the loop and one elected lane issues (elect_one), from descriptors that

@@ -39,20 +39,22 @@
 //                dS, 16-bit operands to TMEM; at the end of an item conversion of the
 //                accumulators.
 //   warps 8-15   the same for odd steps.
-//   warps 16, 17 lane 0 issues the product MMAs of even / odd steps.
-//   warps 18, 19 lane 0 issues the accumulating MMAs, one accumulator each (dV and dK; the
+//   warps 16, 17 issue the product MMAs of even / odd steps.
+//   warps 18, 19 issue the accumulating MMAs, one accumulator each (dV and dK; the
 //                dQ kernel uses warp 18 only), every step in order.
-//   warp 20      lane 0 issues the TMA loads: stationary tiles (two buffers at d_head 64, so
+//   warp 20      issues the TMA loads: stationary tiles (two buffers at d_head 64, so
 //                the next item's arrive early) and the streamed stages.
 //   warp 21      allocates TMEM; at d_head 64 it also issues the TMA stores of the output
 //                tiles, which the compute warps stage in the stationary buffer the finished
 //                item no longer needs (row-strided stores straight from registers cost an L2
 //                write transaction per 16 or 32 bytes and took 1300-2800 clocks per item).
-// An MMA costs its issuing thread 55-110 clocks whatever its size, and two threads issue twice
-// as many (measured), so every MMA stream has a thread of its own; and the per-step waits of
-// a compute warp (products ready, operand columns free, stores complete) are latencies that
-// only other warps' work can fill, hence sixteen compute warps on two steps rather than
-// eight on one.
+// Every MMA stream has a warp of its own, whose loop the whole warp walks while one elected lane
+// (elect_one) issues, from descriptors that differ by constants: with a loop of lane 0 alone, and
+// role and TMEM base not known to be uniform, an MMA cost its thread 55-110 clocks whatever its
+// size, and f16 D=64 causal B*H=96 S=2048 took 276 us instead of 237, bf16 D=128 causal B*H=32
+// S=4096 531 instead of 471.  The per-step waits of a compute warp (products ready, operand columns
+// free, stores complete) are latencies that only other warps' work can fill, hence sixteen compute
+// warps on two steps rather than eight on one.
 #include <cmath>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -218,7 +220,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the shuffles tell the compiler that the role and the TMEM base are the same in the whole warp
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t b_s = base + NA * 2 * L::kTile;        // stationary buffers first, then the stages
     WaitCtl ctl{&abort_flag, status};
@@ -243,123 +246,129 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     if (warp >= kComputeWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsRest));
 
     // gs: steps of the items this CTA has finished; a step's place in every ring is gs + t
     if (warp == kLoadWarp) {
-        // ------------------------------------------------------------ TMA loads (one thread)
-        if (lane == 0) {
-            BwdItem it;
-            int gs = 0;
-            bool ok = true;
-            for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
-                const int buf = k % NA, use = k / NA;
-                // the stationary tiles of item k - NA were last read by its products; where that item's
-                // output was staged in the same buffer, by the TMA store of that output
-                if (use >= 1 && !mbar_wait(smem_u32(STAGED ? &bar_ofree[buf] : &bar_afree[buf]), (use - 1) & 1, ctl, kBwdBarFree)) break;
-                const uint32_t a0_s = base + buf * 2 * L::kTile, a1_s = a0_s + L::kTile;
+        // ------------------------------------------------------------ TMA loads (one elected lane)
+        BwdItem it;
+        int gs = 0;
+        bool ok = true;
+        for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
+            const int buf = k % NA, use = k / NA;
+            // the stationary tiles of item k - NA were last read by its products; where that item's
+            // output was staged in the same buffer, by the TMA store of that output
+            if (use >= 1 && !mbar_wait(smem_u32(STAGED ? &bar_ofree[buf] : &bar_afree[buf]), (use - 1) & 1, ctl, kBwdBarFree)) break;
+            const uint32_t a0_s = base + buf * 2 * L::kTile, a1_s = a0_s + L::kTile;
+            if (elect_one()) {
                 mbar_arrive_expect_tx(smem_u32(&bar_a[buf]), 2 * L::kTile);
                 for (int b = 0; b < NBOX; b++) {
                     tma_load_3d(a0_s + b * L::kBox, &ta0, smem_u32(&bar_a[buf]), b * 64, it.tile * kT, it.bh);
                     tma_load_3d(a1_s + b * L::kBox, &ta1, smem_u32(&bar_a[buf]), b * 64, it.tile * kT, it.bh);
                 }
-                for (int t = 0; t < it.n_steps; t++) {
-                    const int T = gs + t, s = T % kStages;
-                    // the stage held step T - kStages: its accumulations must have completed
-                    if (T >= kStages && !mbar_wait(smem_u32(&bar_acc[s]), ((T - kStages) / kStages) & 1, ctl, kBwdBarFree)) { ok = false; break; }
-                    const uint32_t dst = b_s + s * 2 * L::kTileB;
+            }
+            __syncwarp();
+            for (int t = 0; t < it.n_steps; t++) {
+                const int T = gs + t, s = T % kStages;
+                // the stage held step T - kStages: its accumulations must have completed
+                if (T >= kStages && !mbar_wait(smem_u32(&bar_acc[s]), ((T - kStages) / kStages) & 1, ctl, kBwdBarFree)) { ok = false; break; }
+                const uint32_t dst = b_s + s * 2 * L::kTileB;
+                if (elect_one()) {
                     mbar_arrive_expect_tx(smem_u32(&bar_full[s]), 2 * L::kTileB);
                     for (int b = 0; b < NBOX; b++) {
                         tma_load_3d(dst + b * L::kBoxB, &tb0, smem_u32(&bar_full[s]), b * 64, it.row0 + t * kW, it.bh);
                         tma_load_3d(dst + L::kTileB + b * L::kBoxB, &tb1, smem_u32(&bar_full[s]), b * 64, it.row0 + t * kW, it.bh);
                     }
                 }
-                gs += it.n_steps;
+                __syncwarp();
             }
+            gs += it.n_steps;
         }
-        __syncwarp();
     } else if (warp == kProdWarp || warp == kProdWarp + 1) {
-        // ------------------------------------------------------------ product MMAs of one parity (one thread)
-        if (lane == 0) {
-            const int g = warp - kProdWarp;
-            constexpr uint32_t idesc_t = make_idesc(kT, kW, FMT, FMT, kMajorK, kMajorK);
-            constexpr uint64_t hi_k = make_sdesc_hi(16, 1024);
-            const uint32_t tb = tmem + g * 128;
-            BwdItem it;
-            int gs = 0;
-            bool ok = true;
-            for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
-                const int buf = k % NA, use = k / NA;
-                const uint32_t a0_s = base + buf * 2 * L::kTile, a1_s = a0_s + L::kTile;
-                if (!mbar_wait(smem_u32(&bar_a[buf]), use & 1, ctl, kBwdBarA)) break;
-                bool issued = false;
-                for (int t = (g ^ gs) & 1; t < it.n_steps; t += 2) {
-                    const int T = gs + t, s = T % kStages;
-                    const uint32_t b0_s = b_s + s * 2 * L::kTileB, b1_s = b0_s + L::kTileB;
-                    // the tiles arrived long ago; the buffer is what the issue waits for
-                    if (!mbar_wait(smem_u32(&bar_full[s]), (T / kStages) & 1, ctl, kBwdBarFull)) { ok = false; break; }
-                    if (T >= 2) {
-                        // products of step T reuse the TMEM buffer of step T-2
-                        if (INPLACE) ok = mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
-                        else         ok = mbar_wait(smem_u32(&bar_tfree[g]), ((T >> 1) - 1) & 1, ctl, kBwdBarFree);
-                        if (!ok) break;
-                    }
-                    tc_fence_after();
+        // ------------------------------------------------------------ product MMAs of one parity (one elected lane)
+        const int g = warp - kProdWarp;
+        constexpr uint32_t idesc_t = make_idesc(kT, kW, FMT, FMT, kMajorK, kMajorK);
+        constexpr uint64_t hi_k = make_sdesc_hi(16, 1024);
+        const uint32_t tb = tmem + g * 128;
+        BwdItem it;
+        int gs = 0;
+        bool ok = true;
+        for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
+            const int buf = k % NA, use = k / NA;
+            const uint64_t da0 = make_sdesc(base + buf * 2 * L::kTile, hi_k), da1 = da0 + (L::kTile >> 4);
+            if (!mbar_wait(smem_u32(&bar_a[buf]), use & 1, ctl, kBwdBarA)) break;
+            bool issued = false;
+            for (int t = (g ^ gs) & 1; t < it.n_steps; t += 2) {
+                const int T = gs + t, s = T % kStages;
+                // the tiles arrived long ago; the buffer is what the issue waits for
+                if (!mbar_wait(smem_u32(&bar_full[s]), (T / kStages) & 1, ctl, kBwdBarFull)) { ok = false; break; }
+                if (T >= 2) {
+                    // products of step T reuse the TMEM buffer of step T-2
+                    if (INPLACE) ok = mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
+                    else         ok = mbar_wait(smem_u32(&bar_tfree[g]), ((T >> 1) - 1) & 1, ctl, kBwdBarFree);
+                    if (!ok) break;
+                }
+                tc_fence_after();
+                const uint64_t db0 = make_sdesc(b_s + s * 2 * L::kTileB, hi_k), db1 = db0 + (L::kTileB >> 4);
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
-                        const uint32_t offa = (kk >> 2) * L::kBox + (kk & 3) * 32, offb = (kk >> 2) * L::kBoxB + (kk & 3) * 32;
-                        mma_f16_ss(tb, make_sdesc(a0_s + offa, hi_k), make_sdesc(b0_s + offb, hi_k), idesc_t, kk > 0);
+                        const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
+                        mma_f16_ss(tb, da0 + offa, db0 + offb, idesc_t, kk > 0);
                     }
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
-                        const uint32_t offa = (kk >> 2) * L::kBox + (kk & 3) * 32, offb = (kk >> 2) * L::kBoxB + (kk & 3) * 32;
-                        mma_f16_ss(tb + kW, make_sdesc(a1_s + offa, hi_k), make_sdesc(b1_s + offb, hi_k), idesc_t, kk > 0);
+                        const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
+                        mma_f16_ss(tb + kW, da1 + offa, db1 + offb, idesc_t, kk > 0);
                     }
                     tc_commit(smem_u32(&bar_t[g]));
-                    issued = true;
                 }
-                if (!ok) break;
-                // this parity no longer reads the item's stationary tiles once its products are done
+                __syncwarp();
+                issued = true;
+            }
+            if (!ok) break;
+            // this parity no longer reads the item's stationary tiles once its products are done
+            if (elect_one()) {
                 if (issued) tc_commit(smem_u32(&bar_afree[buf]));
                 else        mbar_arrive(smem_u32(&bar_afree[buf]));
-                gs += it.n_steps;
             }
+            __syncwarp();
+            gs += it.n_steps;
         }
-        __syncwarp();
     } else if (warp == kAccWarp || (warp == kAccWarp + 1 && MODE == 0)) {
-        // ------------------------------------------------------------ accumulating MMAs of one accumulator (one thread)
-        if (lane == 0) {
-            const int x = warp - kAccWarp;
-            constexpr uint32_t idesc_acc = make_idesc(kT, D, FMT, FMT, kMajorK, kMajorMN);
-            constexpr uint64_t hi_mn = make_sdesc_hi(L::kBoxB, 1024);
-            // MODE 0: warp 18 dV += P^T dO (operand P^T, streamed dO = B1), warp 19 dK += dS^T Q (dS^T, Q = B0)
-            // MODE 1: warp 18 dQ += dS K (dS, K = B0)
-            const bool use_p = (MODE == 0 && x == 0);
-            const uint32_t acc = tmem + (x == 0 ? ACC0_COL : ACC1_COL);
-            const uint32_t op0 = tmem + (use_p ? OPP0 : OPD0);
-            BwdItem it;
-            int gs = 0;
-            bool ok = true;
-            for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
-                for (int t = 0; t < it.n_steps; t++) {
-                    const int T = gs + t, s = T % kStages, g = T & 1;
-                    const uint32_t bt_s = b_s + s * 2 * L::kTileB + (use_p ? L::kTileB : 0);
-                    if (!mbar_wait(smem_u32(&bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP)) { ok = false; break; }
-                    // the accumulators of the item before must have been read out
-                    if (t == 0 && k >= 1 && !mbar_wait(smem_u32(&bar_accfree), (k - 1) & 1, ctl, kBwdBarFree)) { ok = false; break; }
-                    tc_fence_after();
+        // ------------------------------------------------------------ accumulating MMAs of one accumulator (one elected lane)
+        const int x = warp - kAccWarp;
+        constexpr uint32_t idesc_acc = make_idesc(kT, D, FMT, FMT, kMajorK, kMajorMN);
+        constexpr uint64_t hi_mn = make_sdesc_hi(L::kBoxB, 1024);
+        // MODE 0: warp 18 dV += P^T dO (operand P^T, streamed dO = B1), warp 19 dK += dS^T Q (dS^T, Q = B0)
+        // MODE 1: warp 18 dQ += dS K (dS, K = B0)
+        const bool use_p = (MODE == 0 && x == 0);
+        const uint32_t acc = tmem + (x == 0 ? ACC0_COL : ACC1_COL);
+        const uint32_t op0 = tmem + (use_p ? OPP0 : OPD0);
+        BwdItem it;
+        int gs = 0;
+        bool ok = true;
+        for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
+            for (int t = 0; t < it.n_steps; t++) {
+                const int T = gs + t, s = T % kStages, g = T & 1;
+                if (!mbar_wait(smem_u32(&bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP)) { ok = false; break; }
+                // the accumulators of the item before must have been read out
+                if (t == 0 && k >= 1 && !mbar_wait(smem_u32(&bar_accfree), (k - 1) & 1, ctl, kBwdBarFree)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t db = make_sdesc(b_s + s * 2 * L::kTileB + (use_p ? L::kTileB : 0), hi_mn);
+                const uint32_t op = op0 + g * OP_STRIDE;
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < kW / 16; kk++)
-                        mma_f16_ts(acc, op0 + g * OP_STRIDE + op16_col(kk, INPLACE), make_sdesc(bt_s + kk * 2048, hi_mn), idesc_acc,
-                                   (t > 0 || kk > 0) ? 1u : 0u);
+                        mma_f16_ts(acc, op + op16_col(kk, INPLACE), db + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
                     tc_commit(smem_u32(&bar_acc[s]));
                     if (t == it.n_steps - 1) tc_commit(smem_u32(&bar_done));
                 }
-                gs += it.n_steps;
+                __syncwarp();
             }
+            gs += it.n_steps;
         }
-        __syncwarp();
     } else if (warp == kTmemWarp && STAGED) {
         // ------------------------------------------------------------ TMA stores of the staged output tiles
         BwdItem it;

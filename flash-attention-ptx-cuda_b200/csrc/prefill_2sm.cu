@@ -116,8 +116,9 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rank = cluster_ctarank();              // 0 = leader (issues the pair's MMAs)
+    // the shuffles tell the compiler that role, rank and TMEM base are the same in the whole warp
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);              // 0 = leader (issues the pair's MMAs)
     const bool leader = rank == 0;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t q_s = base;
@@ -147,7 +148,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     tc_fence_before();
     cluster_sync_all();                                   // both CTAs' barriers and TMEM exist before anyone uses them
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const int G = gridDim.x >> 1;
     const int n_rounds = (n_items + G - 1) / G;
     // the leader's barriers that the peer signals
@@ -160,7 +161,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
     if (warp == 8) {
         // ------------------------------------------------------------ TMA producer: Q and the K halves
-        if (lane == 0) {
+        {
             int g = 0, it_n = 0, g_item0 = 0;
             bool ok = true;
             for (int r = 0; ok && r < n_rounds; r++) {
@@ -168,18 +169,24 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (!get_item2<CAUSAL>(r, n_items, n_bh, n_pairs, seq_len, heads_per_group, it)) continue;
                 // Q is free after the previous item's last Q K^T (entry of that tile in the ring)
                 if (it_n > 0 && !mbar_wait(smem_u32(&bar_qk[(g_item0 - 1) % kRing]), ((g_item0 - 1) / kRing) & 1, ctl, k2QFree)) break;
-                if (leader) mbar_arrive_expect_tx(smem_u32(&bar_qf), 2 * L::kQBytes);    // both CTAs' query tiles
-                for (int b = 0; b < NBOX; b++)
-                    tma_load_3d_2sm(q_s + b * L::kBox, &tm_q, smem_u32(&bar_qf), b * 64,
-                                    (2 * it.pair + static_cast<int>(rank)) * kBM, it.bh);
+                if (elect_one()) {
+                    if (leader) mbar_arrive_expect_tx(smem_u32(&bar_qf), 2 * L::kQBytes);    // both CTAs' query tiles
+                    for (int b = 0; b < NBOX; b++)
+                        tma_load_3d_2sm(q_s + b * L::kBox, &tm_q, smem_u32(&bar_qf), b * 64,
+                                        (2 * it.pair + static_cast<int>(rank)) * kBM, it.bh);
+                }
+                __syncwarp();
                 for (int j = 0; j < it.n_kv; j++, g++) {
                     const int sk = g % kStages;
                     // the slot was last read by Q K^T of tile g - kStages
                     if (g >= kStages && !mbar_wait(smem_u32(&bar_qk[(g - kStages) % kRing]), ((g - kStages) / kRing) & 1, ctl, k2KFree)) { ok = false; break; }
-                    if (leader) mbar_arrive_expect_tx(smem_u32(&bar_kf[sk]), 2 * L::kKHalf);
-                    for (int b = 0; b < NBOX; b++)       // this CTA's 64 keys of the tile
-                        tma_load_3d_2sm(k_s + sk * L::kKHalf + b * (64 * 128), &tm_k, smem_u32(&bar_kf[sk]), b * 64,
-                                        j * kBN + static_cast<int>(rank) * 64, it.bh);
+                    if (elect_one()) {
+                        if (leader) mbar_arrive_expect_tx(smem_u32(&bar_kf[sk]), 2 * L::kKHalf);
+                        for (int b = 0; b < NBOX; b++)   // this CTA's 64 keys of the tile
+                            tma_load_3d_2sm(k_s + sk * L::kKHalf + b * (64 * 128), &tm_k, smem_u32(&bar_kf[sk]), b * 64,
+                                            j * kBN + static_cast<int>(rank) * 64, it.bh);
+                    }
+                    __syncwarp();
                 }
                 it_n++;
                 g_item0 = g;
@@ -188,7 +195,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         __syncwarp();
     } else if (warp == 11) {
         // ------------------------------------------------------------ TMA producer: the V halves
-        if (lane == 0) {
+        {
             int g = 0;
             bool ok = true;
             for (int r = 0; ok && r < n_rounds; r++) {
@@ -197,19 +204,23 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 for (int j = 0; j < it.n_kv; j++, g++) {
                     const int sv = g % kStages;
                     if (g >= kStages && !mbar_wait(smem_u32(&bar_pvd[(g - kStages) % kRing]), ((g - kStages) / kRing) & 1, ctl, k2VFree)) { ok = false; break; }
-                    if (leader) mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), 2 * L::kVHalf);
-                    // this CTA's 64 head-dim columns of the tile's 128 keys
-                    tma_load_3d_2sm(v_s + sv * L::kVHalf, &tm_v, smem_u32(&bar_vf[sv]), static_cast<int>(rank) * 64,
-                                    j * kBN, it.bh);
+                    if (elect_one()) {
+                        if (leader) mbar_arrive_expect_tx(smem_u32(&bar_vf[sv]), 2 * L::kVHalf);
+                        // this CTA's 64 head-dim columns of the tile's 128 keys
+                        tma_load_3d_2sm(v_s + sv * L::kVHalf, &tm_v, smem_u32(&bar_vf[sv]), static_cast<int>(rank) * 64,
+                                        j * kBN, it.bh);
+                    }
+                    __syncwarp();
                 }
             }
         }
         __syncwarp();
     } else if (warp == 9) {
         // ------------------------------------------------------------ Q K^T issuer (leader CTA only)
-        if (leader && lane == 0) {
+        if (leader) {
             constexpr uint32_t idesc_qk = make_idesc(2 * kBM, kBN, FMT, FMT, kMajorK, kMajorK);
             constexpr uint64_t hi_k = make_sdesc_hi(16, 1024);
+            const uint64_t dq = make_sdesc(q_s, hi_k);
             int g = 0, it_n = 0, u = 0;
             bool ok = true;
             for (int r = 0; ok && r < n_rounds; r++) {
@@ -222,15 +233,18 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     // the score buffer last held S and then P of tile g - kNU: that P V must be done
                     if (g >= kNU && !mbar_wait(smem_u32(&bar_pvd[(g - kNU) % kRing]), ((g - kNU) / kRing) & 1, ctl, k2SFree)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t kb = k_s + sk * L::kKHalf;
+                    const uint64_t dk = make_sdesc(k_s + sk * L::kKHalf, hi_k);
                     const uint32_t sc = tmem + u * 128;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < D / 16; kk++) {
-                        const uint32_t qoff = (kk >> 2) * L::kBox + (kk & 3) * 32;
-                        const uint32_t koff = (kk >> 2) * (64 * 128) + (kk & 3) * 32;
-                        mma_f16_ss_2sm(sc, make_sdesc(q_s + qoff, hi_k), make_sdesc(kb + koff, hi_k), idesc_qk, kk > 0);
+                        for (int kk = 0; kk < D / 16; kk++) {
+                            const uint32_t qoff = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4;
+                            const uint32_t koff = ((kk >> 2) * (64 * 128) + (kk & 3) * 32) >> 4;
+                            mma_f16_ss_2sm(sc, dq + qoff, dk + koff, idesc_qk, kk > 0);
+                        }
+                        tc_commit_2sm(smem_u32(&bar_qk[g % kRing]));  // both CTAs: S ready, K slot free, (last tile) Q free
                     }
-                    tc_commit_2sm(smem_u32(&bar_qk[g % kRing]));      // both CTAs: S ready, K slot free, (last tile) Q free
+                    __syncwarp();
                     u = (u == kNU - 1) ? 0 : u + 1;
                 }
                 it_n++;
@@ -239,7 +253,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         __syncwarp();
     } else if (warp == 10) {
         // ------------------------------------------------------------ P V issuer (leader CTA only)
-        if (leader && lane == 0) {
+        if (leader) {
             constexpr uint32_t idesc_pv = make_idesc(2 * kBM, D, FMT, FMT, kMajorK, kMajorMN);
             constexpr uint64_t hi_v = make_sdesc_hi(L::kBox, 1024);
             int g = 0, it_n = 0, u = 0, u_phase = 0;
@@ -254,13 +268,15 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     // the first P V of an item overwrites O: both CTAs' epilogues must have read the previous one
                     if (j == 0 && it_n > 0 && !mbar_wait_cluster(smem_u32(&bar_ofree), (it_n - 1) & 1, ctl, k2OFree)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t vb = v_s + sv * L::kVHalf;
+                    const uint64_t dv = make_sdesc(v_s + sv * L::kVHalf, hi_v);
                     const uint32_t pc = tmem + u * 128;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < kBN / 16; kk++)
-                        mma_f16_ts_2sm(tmem + O_COL, pc + kk * 8, make_sdesc(vb + kk * 2048, hi_v), idesc_pv,
-                                       (j > 0 || kk > 0) ? 1u : 0u);
-                    tc_commit_2sm(smem_u32(&bar_pvd[g % kRing]));     // both CTAs: score buffer and V slot free, (last tile) O done
+                        for (int kk = 0; kk < kBN / 16; kk++)
+                            mma_f16_ts_2sm(tmem + O_COL, pc + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                        tc_commit_2sm(smem_u32(&bar_pvd[g % kRing])); // both CTAs: score buffer and V slot free, (last tile) O done
+                    }
+                    __syncwarp();
                     if (u == kNU - 1) { u = 0; u_phase ^= 1; } else { u++; }
                 }
                 it_n++;

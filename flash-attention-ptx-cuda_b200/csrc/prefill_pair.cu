@@ -196,7 +196,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
     extern __shared__ uint8_t smem_raw[];
     PairCtrl& cb = *reinterpret_cast<PairCtrl*>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the shuffles tell the compiler that the role and the TMEM base are the same in the whole warp
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const uint32_t base = (smem_u32(smem_raw) + L::kCtrl + 1023u) & ~1023u;
     const uint32_t q_s = base;                            // Q_A, Q_B
     const uint32_t k_s = q_s + 2 * L::kTile;
@@ -234,7 +235,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = cb.tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, cb.tmem_slot, 0);
     const int n_rounds = (n_items + gridDim.x - 1) / gridDim.x;
     // waits until product `t` of query tile X has completed (t < 0: nothing to wait for)
     auto wait_qk_done = [&](int X, int t, int id) -> bool {
@@ -257,7 +258,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // ------------------------------------------------------------ TMA producer(s)
         const bool do_k = warp == kWarpLoadKV;            // Q and K
         const bool do_v = warp == kWarpLoadV;
-        if (lane == 0) {
+        {
             int g = 0, it_a = 0, it_b = 0;                // K/V tiles loaded; items seen with a tile A / B
             int t_a = 0, t_b = 0;                         // key tiles of query tile A / B before this item
             // per ring slot: the chain tiles (A's and B's count, -1 = none) whose product last read it
@@ -273,24 +274,33 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                             // Q_A goes first: with K(0) it is all the item's first Q K^T needs.  The
                             // buffer is free after the previous item's last Q K^T of this query tile.
                             if (!wait_qk_done(0, t_a - 1, kPQFree)) { ok = false; break; }
-                            mbar_arrive_expect_tx(smem_u32(&cb.q_full[0]), L::kTile);
-                            for (int b = 0; b < NBOX; b++)
-                                tma_load_3d(q_s + b * L::kBox, &tm_q, smem_u32(&cb.q_full[0]), b * 64, it.qa, it.bh);
+                            if (elect_one()) {
+                                mbar_arrive_expect_tx(smem_u32(&cb.q_full[0]), L::kTile);
+                                for (int b = 0; b < NBOX; b++)
+                                    tma_load_3d(q_s + b * L::kBox, &tm_q, smem_u32(&cb.q_full[0]), b * 64, it.qa, it.bh);
+                            }
+                            __syncwarp();
                             it_a++;
                         }
                         const int sk = g % NK;
                         if (g >= NK && !(wait_qk_done(0, k_user[0][sk], kPKFree) && wait_qk_done(1, k_user[1][sk], kPKFree))) { ok = false; break; }
                         k_user[0][sk] = ua; k_user[1][sk] = ub;
-                        mbar_arrive_expect_tx(smem_u32(&cb.k_full[sk]), L::kTile);
-                        for (int b = 0; b < NBOX; b++)
-                            tma_load_3d(k_s + sk * L::kTile + b * L::kBox, &tm_k, smem_u32(&cb.k_full[sk]), b * 64,
-                                        j * kBN, it.bh);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(smem_u32(&cb.k_full[sk]), L::kTile);
+                            for (int b = 0; b < NBOX; b++)
+                                tma_load_3d(k_s + sk * L::kTile + b * L::kBox, &tm_k, smem_u32(&cb.k_full[sk]), b * 64,
+                                            j * kBN, it.bh);
+                        }
+                        __syncwarp();
                         if (j == 0 && it.n_b > 0) {
                             if (!wait_qk_done(1, t_b - 1, kPQFree)) { ok = false; break; }
-                            mbar_arrive_expect_tx(smem_u32(&cb.q_full[1]), L::kTile);
-                            for (int b = 0; b < NBOX; b++)
-                                tma_load_3d(q_s + L::kTile + b * L::kBox, &tm_q, smem_u32(&cb.q_full[1]), b * 64,
-                                            it.qa + kBM, it.bh);
+                            if (elect_one()) {
+                                mbar_arrive_expect_tx(smem_u32(&cb.q_full[1]), L::kTile);
+                                for (int b = 0; b < NBOX; b++)
+                                    tma_load_3d(q_s + L::kTile + b * L::kBox, &tm_q, smem_u32(&cb.q_full[1]), b * 64,
+                                                it.qa + kBM, it.bh);
+                            }
+                            __syncwarp();
                             it_b++;
                         }
                     }
@@ -298,10 +308,13 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                         const int sv = g % NV;
                         if (g >= NV && !(wait_pv_done(0, v_user[0][sv], kPVFree) && wait_pv_done(1, v_user[1][sv], kPVFree))) { ok = false; break; }
                         v_user[0][sv] = ua; v_user[1][sv] = ub;
-                        mbar_arrive_expect_tx(smem_u32(&cb.v_full[sv]), L::kTile);
-                        for (int b = 0; b < NBOX; b++)
-                            tma_load_3d(v_s + sv * L::kTile + b * L::kBox, &tm_v, smem_u32(&cb.v_full[sv]), b * 64,
-                                        j * kBN, it.bh);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(smem_u32(&cb.v_full[sv]), L::kTile);
+                            for (int b = 0; b < NBOX; b++)
+                                tma_load_3d(v_s + sv * L::kTile + b * L::kBox, &tm_v, smem_u32(&cb.v_full[sv]), b * 64,
+                                            j * kBN, it.bh);
+                        }
+                        __syncwarp();
                     }
                 }
                 t_a += it.n_a; t_b += it.n_b;
@@ -310,10 +323,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         __syncwarp();
     } else if (warp == kWarpChainA || warp == kWarpChainB) {
         // ------------------------------------------------------------ MMA issuers
-        // One thread (lane 0) runs its whole loop.  (Measured in isolation: one thread issuing back
-        // to back needs ~55-63 clocks per tcgen05.mma, a warp-uniform loop with a predicated issue
-        // per instruction ~70-76; next to busy softmax warps about 100.)
-        if (lane == 0) {
+        // The whole warp walks the loop and one elected lane issues (elect_one).
+        {
         constexpr uint32_t idesc_qk = make_idesc(kBM, kBN, FMT, FMT, kMajorK, kMajorK);
         constexpr uint32_t idesc_pv = make_idesc(kBM, D, FMT, FMT, kMajorK, kMajorMN);
         constexpr uint64_t hi_k = make_sdesc_hi(16, 1024);
@@ -333,14 +344,17 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
             tc_fence_after();
             FA_PROBE(1);
-            const uint32_t kb = k_s + sk * L::kTile, qx_s = q_s + X * L::kTile;
+            const uint64_t dk = make_sdesc(k_s + sk * L::kTile, hi_k), dq = make_sdesc(q_s + X * L::kTile, hi_k);
             const uint32_t s_t = tmem + (X ? S_COL1 : S_COL0);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < D / 16; kk++) {
-                const uint32_t off = (kk >> 2) * L::kBox + (kk & 3) * 32;
-                mma_f16_ss(s_t, make_sdesc(qx_s + off, hi_k), make_sdesc(kb + off, hi_k), idesc_qk, kk > 0);
+                for (int kk = 0; kk < D / 16; kk++) {
+                    const uint32_t off = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4;
+                    mma_f16_ss(s_t, dq + off, dk + off, idesc_qk, kk > 0);
+                }
+                tc_commit(smem_u32(&cb.s_full[X][(t[X] + j) % kRing]));
             }
-            tc_commit(smem_u32(&cb.s_full[X][(t[X] + j) % kRing]));
+            __syncwarp();
             FA_PROBE(2);
             return true;
         };
@@ -355,12 +369,15 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (j == 0 && itx[X] > 0 && !mbar_wait(smem_u32(&cb.o_free[X]), (itx[X] - 1) & 1, ctl, kPOFree)) return false;
             tc_fence_after();
             FA_PROBE(5);
-            const uint32_t vb = v_s + sv * L::kTile;
+            const uint64_t dv = make_sdesc(v_s + sv * L::kTile, hi_v);
             const uint32_t p_t = tmem + (X ? P_COL1 : P_COL0), o_t = tmem + (X ? O_COL1 : O_COL0);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kBN / 16; kk++)
-                mma_f16_ts(o_t, p_t + kk * 8, make_sdesc(vb + kk * 2048, hi_v), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-            tc_commit(smem_u32(&cb.pv_done[X][(t[X] + j) % kRing]));
+                for (int kk = 0; kk < kBN / 16; kk++)
+                    mma_f16_ts(o_t, p_t + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                tc_commit(smem_u32(&cb.pv_done[X][(t[X] + j) % kRing]));
+            }
+            __syncwarp();
             FA_PROBE(6);
             return true;
         };

@@ -54,6 +54,7 @@
 // (SPLIT: two accumulators, [384,448) and [448,512)).
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 
 #include "fast_div.h"
 #include "host_common.h"
@@ -318,28 +319,40 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const int n_rounds = (n_items + gridDim.x - 1) / gridDim.x;
 
-    // Grouped-query decode: one 128-key tile of K or V of (batch, KV head) from the cache.  Dense or
-    // strided cache: tensor map (d, key, KV head, batch).  Paged cache: tensor map (d, key in page,
-    // KV head, page); a tile is one box inside a page, or 128 / page_size boxes of one page each;
+    // Grouped-query decode: one 128-key tile of K or V of (batch, KV head) from the cache, issued by a whole
+    // warp.  Dense or strided cache: tensor map (d, key, KV head, batch).  Paged cache: tensor map (d, key
+    // in page, KV head, page); a tile is one box inside a page, or 128 / page_size boxes of one page each;
     // pages past the end of the sequence are fetched at coordinate -1, which reads as zero.
-    auto load_cache_tile = [&](uint32_t dst, const CUtensorMap* tm, uint32_t bar, const Item& it, int j) {
+    // A tile's page numbers come from cache_pages, lane i that of its i-th page, called a tile ahead: read
+    // one by one while issuing they are eight dependent loads a tile (B=16 Hkv=8 Skv<=4096 D=128: 44.2 us,
+    // now 40.2).  The producers have a loop for either kind of cache: a few more instructions
+    // per tile on the other one cost D=128 chunks 3-5 %.
+    auto cache_pages = [&](const Item& it, int j) -> int {
+        const int off = lane << gq.page_shift, rr = (it.t0 + j) * kBN + off;
+        if (off >= kBN || rr >= it.kv_len || j >= it.n_kv) return -1;
+        return __ldg(gq.block_table + static_cast<size_t>(it.b) * gq.table_stride + (rr >> gq.page_shift));
+    };
+    auto load_cache_tile = [&](uint32_t dst, uint32_t bytes, const CUtensorMap* tm, uint32_t bar, const Item& it, int j, int pages, auto paged) {
         constexpr int NB = FP8 ? 1 : NBOX;            // boxes per tile row: e4m3 rows are one 128-byte box
         constexpr int XS = FP8 ? 128 : 64;            // elements per box row
-        const int hkv = it.hkv, b = it.b;
         const int r0 = (it.t0 + j) * kBN;
-        if (gq.block_table == nullptr) {
-            for (int bx = 0; bx < NB; bx++) tma_load_4d(dst + bx * L::kBox, tm, bar, bx * XS, r0, hkv, b);
+        if constexpr (!decltype(paged)::value) {
+            if (elect_one()) {
+                mbar_arrive_expect_tx(bar, bytes);
+                for (int bx = 0; bx < NB; bx++) tma_load_4d(dst + bx * L::kBox, tm, bar, bx * XS, r0, it.hkv, it.b);
+            }
         } else {
+            if (elect_one()) mbar_arrive_expect_tx(bar, bytes);
             const int ps = 1 << gq.page_shift;
             const int rows = min(ps, kBN);            // rows per box
-            const int* tbl = gq.block_table + static_cast<size_t>(b) * gq.table_stride;
             for (int i = 0; i < kBN / rows; i++) {
-                const int rr = r0 + i * rows;
-                const int page = rr < it.kv_len ? __ldg(tbl + (rr >> gq.page_shift)) : -1;
-                for (int bx = 0; bx < NB; bx++)
-                    tma_load_4d(dst + bx * L::kBox + i * rows * 128, tm, bar, bx * XS, rr & (ps - 1), hkv, page);
+                const int page = __shfl_sync(0xffffffffu, pages, i);
+                if (elect_one())
+                    for (int bx = 0; bx < NB; bx++)
+                        tma_load_4d(dst + bx * L::kBox + i * rows * 128, tm, bar, bx * XS, (r0 + i * rows) & (ps - 1), it.hkv, page);
             }
         }
+        __syncwarp();
     };
     if (warp >= 12) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsHelper));
     else if (warp >= 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -351,6 +364,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // a key tile (B=16 Hkv=8 Skv<=4096 D=128 56.7 -> 43.9 us; a [B, S, H, D] cache 38.5 -> 36.2).
         constexpr int NLOAD = FP8 ? 1 : NBOX;             // boxes per Q / K tile
         constexpr int XSTEP = FP8 ? 128 : 64;             // elements per box row
+        auto produce = [&](auto paged) {
         int g = 0, it_n = 0;
         bool ok = true;
         for (int r = 0; ok && r < n_rounds; r++) {
@@ -370,21 +384,25 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
             }
             __syncwarp();
+            int pages = -1;
+            if constexpr (decltype(paged)::value) pages = cache_pages(it, 0);
             for (int j = 0; j < it.n_kv; j++, g++) {
                 const int sk = g % NK;
+                const int pages_j = pages;
+                if constexpr (decltype(paged)::value) pages = cache_pages(it, j + 1);
                 // the slot was last read by Q K^T of tile g - NK
                 if (g >= NK && !mbar_wait(smem_u32(&bar_qk[(g - NK) % kRing]), ((g - NK) / kRing) & 1, ctl, kBarKEmpty)) { ok = false; break; }
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(smem_u32(&bar_kf[sk]), L::kKBytes);
-                    if constexpr (GQA) {
-                        load_cache_tile(k_s + sk * L::kKBytes, &tm_k, smem_u32(&bar_kf[sk]), it, j);
-                    } else {
+                if constexpr (GQA) {
+                    load_cache_tile(k_s + sk * L::kKBytes, L::kKBytes, &tm_k, smem_u32(&bar_kf[sk]), it, j, pages_j, paged);
+                } else {
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(smem_u32(&bar_kf[sk]), L::kKBytes);
                         for (int b = 0; b < NLOAD; b++)
                             tma_load_3d(k_s + sk * L::kKBytes + b * L::kBox, &tm_k, smem_u32(&bar_kf[sk]),
                                         b * XSTEP, j * kBN, it.bh);
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
                 if constexpr (SPLIT) {
                     // V as well (warp 11 issues P V here): with four stages each the V slot, P V of tile
                     // g - 4, frees before Q K^T may use the next K tile, which needs P V of tile g - 2
@@ -400,23 +418,27 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             it_n++;
         }
+        };
+        if (GQA && gq.block_table != nullptr) produce(std::true_type{});
+        else                                  produce(std::false_type{});
     } else if (!SPLIT && warp == 11) {
         // ------------------------------------------------------------ TMA producer: V
+        auto produce = [&](auto paged) {
         int g = 0, n_scrub = 0;
         bool ok = true;
         for (int r = 0; ok && r < n_rounds; r++) {
             Item it;
             if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
+            int pages = -1;
+            if constexpr (decltype(paged)::value) pages = cache_pages(it, 0);
             for (int j = 0; j < it.n_kv; j++, g++) {
+                const int pages_j = pages;
+                if constexpr (decltype(paged)::value) pages = cache_pages(it, j + 1);
                 if constexpr (V8) {
                     // e4m3 V lands in its own buffers; warps 12-15 turn it into the fp16 operand.
                     const int s8 = g & 1;
                     if (g >= 2 && !mbar_wait(smem_u32(&bar_v8e[s8]), ((g >> 1) - 1) & 1, ctl, kBarV8Empty)) { ok = false; break; }
-                    if (elect_one()) {
-                        mbar_arrive_expect_tx(smem_u32(&bar_v8f[s8]), L::kV8Bytes);
-                        load_cache_tile(v8_s + s8 * L::kV8Bytes, &tm_v, smem_u32(&bar_v8f[s8]), it, j);
-                    }
-                    __syncwarp();
+                    load_cache_tile(v8_s + s8 * L::kV8Bytes, L::kV8Bytes, &tm_v, smem_u32(&bar_v8f[s8]), it, j, pages_j, paged);
                 } else {
                     const int sv = g % NV;
                     // the slot was last read by P V of tile g - NV
@@ -431,11 +453,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         const int valid = it.kv_len - (it.t0 + j) * kBN;      // rows of this tile inside the sequence
                         const bool scrub = valid < kBN && (gq.seq_lens != nullptr || gq.block_table != nullptr);
                         const uint32_t full = scrub ? smem_u32(&bar_vraw) : smem_u32(&bar_vf[sv]);
-                        if (elect_one()) {
-                            mbar_arrive_expect_tx(full, L::kVBytes);
-                            load_cache_tile(vdst, &tm_v, full, it, j);
-                        }
-                        __syncwarp();
+                        load_cache_tile(vdst, L::kVBytes, &tm_v, full, it, j, pages_j, paged);
                         if (scrub) {
                             if (!mbar_wait(full, n_scrub & 1, ctl, kBarVFull)) { ok = false; break; }
                             n_scrub++;
@@ -458,6 +476,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
             }
         }
+        };
+        if (GQA && gq.block_table != nullptr) produce(std::true_type{});
+        else                                  produce(std::false_type{});
     } else if (warp == 9) {
         // ------------------------------------------------------------ Q K^T issuer
         // The whole warp walks the loop and one elected lane issues (elect_one), from descriptors that
@@ -628,21 +649,38 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     // decode over a cache: rows past the sequence's end may hold stale bytes (NaN codes
                     // included); they are written as zero so that P = 0 there cannot poison O
                     const int valid = GQA ? it.kv_len - (it.t0 + j) * kBN : kBN;
-#pragma unroll 4
-                    for (int i = 0; i < (kBN * 16) / 128; i++) {
-                        const int c16 = ct + i * 128;         // 8-element group: row c16/16, group-in-row c16%16
-                        const int rr = c16 >> 4, c8 = c16 & 15;
-                        const uint32_t src = src_base + rr * 128 + (((c8 >> 1) ^ (rr & 7)) << 4) + ((c8 & 1) << 3);
-                        uint32_t lo, hi;
-                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(lo), "=r"(hi) : "r"(src));
-                        if (GQA && rr >= valid) { lo = 0u; hi = 0u; }
-                        const uint32_t w0 = e4m3x2_to_f16x2(static_cast<uint16_t>(lo & 0xFFFFu));
-                        const uint32_t w1 = e4m3x2_to_f16x2(static_cast<uint16_t>(lo >> 16));
-                        const uint32_t w2 = e4m3x2_to_f16x2(static_cast<uint16_t>(hi & 0xFFFFu));
-                        const uint32_t w3 = e4m3x2_to_f16x2(static_cast<uint16_t>(hi >> 16));
-                        const uint32_t dst = dst_base + (c8 >> 3) * L::kBox + rr * 128 + (((c8 & 7) ^ (rr & 7)) << 4);
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w0), "r"(w1),
-                                     "r"(w2), "r"(w3) : "memory");
+                    // A thread takes 16 codes (one 16-byte chunk) of eight rows, all loaded before the first is
+                    // used: 8 bytes at a time, a few in flight, the loads' latency made this the slowest role
+                    // of the kernel (B=32 Hkv=8 Skv=16384: 258 us, now 225, and 213 with the loads above changed too).  Codes 16 ch .. 16 ch + 15 become the chunks
+                    // 2 ch and 2 ch + 1 of a 256-byte fp16 row (two boxes of 8 chunks); the threads of the
+                    // second box write their odd chunk first, so that a quarter warp, which covers one row,
+                    // meets every bank once.
+                    const int ch = ct & 7, r0 = ct >> 3;             // chunk; first row (then every 16th)
+                    uint4 c[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int rr = r0 + i * 16;
+                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(c[i].x), "=r"(c[i].y), "=r"(c[i].z), "=r"(c[i].w)
+                                     : "r"(src_base + rr * 128 + ((ch ^ (rr & 7)) << 4)));
+                    }
+                    const bool odd_first = ch >= 4;
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int rr = r0 + i * 16;
+                        if (GQA && rr >= valid) c[i] = make_uint4(0u, 0u, 0u, 0u);
+                        const uint32_t row = dst_base + (ch >> 2) * L::kBox + rr * 128;
+                        const int c0 = (ch & 3) * 2;                  // even chunk of the pair within its box
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const bool hi = (h == 1) != odd_first;    // which half of the 16 codes
+                            const uint32_t a = hi ? c[i].z : c[i].x, b = hi ? c[i].w : c[i].y;
+                            const uint32_t w0 = e4m3x2_to_f16x2(static_cast<uint16_t>(a & 0xFFFFu));
+                            const uint32_t w1 = e4m3x2_to_f16x2(static_cast<uint16_t>(a >> 16));
+                            const uint32_t w2 = e4m3x2_to_f16x2(static_cast<uint16_t>(b & 0xFFFFu));
+                            const uint32_t w3 = e4m3x2_to_f16x2(static_cast<uint16_t>(b >> 16));
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + (((c0 + (hi ? 1 : 0)) ^ (rr & 7)) << 4)),
+                                         "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
+                        }
                     }
                     fence_proxy_async_smem();             // the tensor core reads the copy through the async proxy
                     mbar_arrive(smem_u32(&bar_vf[sv]));

@@ -13,6 +13,8 @@
 //     fp32 accumulator slice) per lane group in registers, and never touches
 //     shared memory until the per-CTA merge at the end.  Output per (head,
 //     split): a normalised fp32 partial O and its natural-log LSE.
+//   decode_cluster_kernel  the same pass when a head needs at most 8 CTAs: they form a thread-block
+//     cluster and merge through distributed shared memory, so that one launch writes the result.
 //   combine_kernel  merges partials by their LSEs,
 //       m = max lse_p, w_p = exp(lse_p - m), O = sum w_p O_p / sum w_p,
 //       LSE = m + log(sum w_p),
@@ -40,6 +42,19 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2   = 0.6931471805599453f;
 constexpr int   kDecodeWarps = 8;
 constexpr int   kUnroll = 4;            // row groups in flight per warp iteration
+constexpr int   kMaxCluster = 8;        // portable cluster size
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The float that CTA `rank` of the cluster has at this CTA's shared address `p`.
+__device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
+    uint32_t addr;
+    float x;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
+    return x;
+}
 
 __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
     uint4 r;
@@ -81,22 +96,23 @@ __device__ __forceinline__ void merge_state(float& m, float& l, float (&acc)[8],
     m = mn;
 }
 
-template <int D, bool BF16>
-__global__ void __launch_bounds__(kDecodeWarps * 32)
-decode_partial_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
-                      const uint16_t* __restrict__ v, float* __restrict__ o_part,
-                      float* __restrict__ lse_part, int seq_len_kv, int n_splits, int keys_per_split,
-                      float scale_log2) {
+// Result of one CTA's keys: running max (log2 units), sum and unnormalised accumulator of thread d < D.
+template <int D, int WARPS>
+struct DecodeShared {
+    float m[WARPS], l[WARPS], acc[WARPS][D];
+};
+
+// Keys [k_begin, k_end) of head bh, by the whole CTA; valid in threads < D.
+template <int D, bool BF16, int WARPS>
+__device__ __forceinline__ void decode_keys(DecodeShared<D, WARPS>& sm, const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
+                                            const uint16_t* __restrict__ v, int bh, int k_begin, int k_end, int seq_len_kv,
+                                            float scale_log2, float& mm, float& ll, float& a) {
     constexpr int LPR = D / 8;           // lanes covering one row (8 elements = 16 bytes per lane)
     constexpr int RPW = 32 / LPR;        // rows per warp-wide load
-    constexpr int STEP = kDecodeWarps * RPW;
-    // one-dimensional grid: the splits of a head are neighbours, and batch * heads is not limited to 65535
-    const int bh = blockIdx.x / n_splits, split = blockIdx.x - bh * n_splits;
+    constexpr int STEP = WARPS * RPW;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / LPR;          // which row of the warp-wide load this lane reads
     const int dsl = (lane % LPR) * 8;    // first of this lane's 8 head-dim elements
-    const int k_begin = split * keys_per_split;
-    const int k_end = min(seq_len_kv, k_begin + keys_per_split);
 
     float qf[8];
     {
@@ -167,56 +183,52 @@ decode_partial_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict
         merge_state(m, l, acc, m2, l2, a2);
     }
     // Merge the warps of the CTA through shared memory.
-    __shared__ float sm_m[kDecodeWarps], sm_l[kDecodeWarps];
-    __shared__ float sm_acc[kDecodeWarps][D];
     if (lane < LPR) {
 #pragma unroll
-        for (int e = 0; e < 8; e++) sm_acc[warp][dsl + e] = acc[e];
-        if (lane == 0) { sm_m[warp] = m; sm_l[warp] = l; }
+        for (int e = 0; e < 8; e++) sm.acc[warp][dsl + e] = acc[e];
+        if (lane == 0) { sm.m[warp] = m; sm.l[warp] = l; }
     }
     __syncthreads();
+    mm = -1e30f;
+    ll = 0.0f;
+    a = 0.0f;
     if (threadIdx.x < D) {
         const int d = threadIdx.x;
-        float mm = -1e30f;
 #pragma unroll
-        for (int w = 0; w < kDecodeWarps; w++) mm = fmaxf(mm, sm_m[w]);
-        float ll = 0.0f, a = 0.0f;
+        for (int w = 0; w < WARPS; w++) mm = fmaxf(mm, sm.m[w]);
 #pragma unroll
-        for (int w = 0; w < kDecodeWarps; w++) {
-            const float c = fast_ex2(sm_m[w] - mm);
-            ll += sm_l[w] * c;
-            a += sm_acc[w][d] * c;
+        for (int w = 0; w < WARPS; w++) {
+            const float c = fast_ex2(sm.m[w] - mm);
+            ll += sm.l[w] * c;
+            a += sm.acc[w][d] * c;
         }
+    }
+}
+
+template <int D, bool BF16>
+__global__ void __launch_bounds__(kDecodeWarps * 32)
+decode_partial_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
+                      const uint16_t* __restrict__ v, float* __restrict__ o_part,
+                      float* __restrict__ lse_part, int seq_len_kv, int n_splits, int keys_per_split,
+                      float scale_log2) {
+    __shared__ DecodeShared<D, kDecodeWarps> sm;
+    // one-dimensional grid: the splits of a head are neighbours, and batch * heads is not limited to 65535
+    const int bh = blockIdx.x / n_splits, split = blockIdx.x - bh * n_splits;
+    const int k_begin = split * keys_per_split;
+    float mm, ll, a;
+    decode_keys<D, BF16, kDecodeWarps>(sm, q, k, v, bh, k_begin, min(seq_len_kv, k_begin + keys_per_split), seq_len_kv, scale_log2, mm, ll, a);
+    if (threadIdx.x < D) {
+        const int d = threadIdx.x;
         const size_t pidx = (size_t)bh * n_splits + split;
         o_part[pidx * D + d] = ll > 0.0f ? a / ll : 0.0f;
         if (d == 0) lse_part[pidx] = ll > 0.0f ? kLn2 * (mm + log2f(ll)) : -INFINITY;
     }
 }
 
-// One CTA per output row, one thread per head-dim element.  Inputs and the fp32 output are
-// addressed by strides, so the same kernel reads split partials ([row][split][D]), gathered
-// per-rank partials ([rank][row][D]) and packed ones ([rank][row][D + 1], LSE in the last
-// column), and can write a packed row itself.
+// A head's output, written by the one thread per head-dim element that holds it.
 template <bool BF16>
-__global__ void combine_kernel(const float* __restrict__ o_parts, const float* __restrict__ lse_parts,
-                               int n_parts, long long part_stride_o, long long row_stride_o,
-                               long long part_stride_l, long long row_stride_l, int d_head,
-                               uint16_t* __restrict__ o, float* __restrict__ lse, long long lse_stride,
-                               float* __restrict__ o_f32, long long o_f32_stride) {
-    const int row = blockIdx.x, d = threadIdx.x;
-    const float* lp = lse_parts + (size_t)row * row_stride_l;
-    float m = -INFINITY;
-    for (int p = 0; p < n_parts; p++) m = fmaxf(m, lp[(size_t)p * part_stride_l]);
-    float wsum = 0.0f, a = 0.0f;
-    if (m > -INFINITY) {
-        const float* op = o_parts + (size_t)row * row_stride_o + d;
-        for (int p = 0; p < n_parts; p++) {
-            const float w = fast_ex2((lp[(size_t)p * part_stride_l] - m) * kLog2e);
-            wsum += w;
-            a = fmaf(w, op[(size_t)p * part_stride_o], a);
-        }
-    }
-    const float out = wsum > 0.0f ? a / wsum : 0.0f;
+__device__ __forceinline__ void write_row(int row, int d, int d_head, float out, float lse_val, uint16_t* o, float* lse,
+                                          long long lse_stride, float* o_f32, long long o_f32_stride) {
     if (o != nullptr) {
         uint16_t bits;
         if constexpr (BF16) bits = __bfloat16_as_ushort(__float2bfloat16_rn(out));
@@ -224,7 +236,105 @@ __global__ void combine_kernel(const float* __restrict__ o_parts, const float* _
         o[(size_t)row * d_head + d] = bits;
     }
     if (o_f32 != nullptr) o_f32[(size_t)row * o_f32_stride + d] = out;
-    if (lse != nullptr && d == 0) lse[(size_t)row * lse_stride] = wsum > 0.0f ? m + kLn2 * log2f(wsum) : -INFINITY;
+    if (lse != nullptr && d == 0) lse[(size_t)row * lse_stride] = lse_val;
+}
+
+// Decode with the CTAs of a head as one cluster (1 to 8 of them, gridDim.x = heads x cluster size):
+// every CTA takes a slice of the keys, the merge reads the CTAs' results through distributed shared memory
+// and the first CTA writes the output.  No partials in memory and no second kernel, so what a short
+// job waits for is one launch and one pass of loads.  Per call in a graph: bf16 D=64 B*H=24 Skv=1537
+// 7.0 -> 4.5 us, f16 D=128 B*H=32 Skv=512 8.2 -> 3.9, Skv=4096 18.0 -> 16.5.
+template <int D, bool BF16, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+decode_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k, const uint16_t* __restrict__ v,
+                      int seq_len_kv, int n_ctas, int keys_per_cta, float scale_log2, uint16_t* __restrict__ o,
+                      float* __restrict__ lse, long long lse_stride, float* __restrict__ o_f32, long long o_f32_stride) {
+    __shared__ DecodeShared<D, WARPS> sm;
+    __shared__ float res_a[D], res_m, res_l;
+    const int bh = blockIdx.x / n_ctas, rank = blockIdx.x - bh * n_ctas;
+    const int k_begin = min(seq_len_kv, rank * keys_per_cta);
+    float mm, ll, a;
+    decode_keys<D, BF16, WARPS>(sm, q, k, v, bh, k_begin, min(seq_len_kv, k_begin + keys_per_cta), seq_len_kv, scale_log2, mm, ll, a);
+    const int d = threadIdx.x;
+    if (n_ctas > 1) {
+        if (d < D) res_a[d] = a;
+        if (d == 0) { res_m = mm; res_l = ll; }
+        cluster_barrier();                                // every CTA's result is in its shared memory
+        if (rank == 0 && d < D) {
+            float pm[kMaxCluster], pl[kMaxCluster], pa[kMaxCluster];
+            mm = -1e30f;
+#pragma unroll
+            for (int c = 0; c < kMaxCluster; c++) {
+                pm[c] = -1e30f; pl[c] = 0.0f; pa[c] = 0.0f;
+                if (c < n_ctas) {
+                    pm[c] = ld_cluster_f32(&res_m, c);
+                    pl[c] = ld_cluster_f32(&res_l, c);
+                    pa[c] = ld_cluster_f32(&res_a[d], c);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < kMaxCluster; c++) mm = fmaxf(mm, pm[c]);
+            ll = 0.0f;
+            a = 0.0f;
+#pragma unroll
+            for (int c = 0; c < kMaxCluster; c++) {
+                const float w = fast_ex2(pm[c] - mm);
+                ll = fmaf(pl[c], w, ll);
+                a = fmaf(pa[c], w, a);
+            }
+        }
+        cluster_barrier();                                // nobody leaves while its shared memory may be read
+    }
+    if (rank == 0 && d < D)
+        write_row<BF16>(bh, d, D, ll > 0.0f ? a / ll : 0.0f, ll > 0.0f ? kLn2 * (mm + log2f(ll)) : -INFINITY, o, lse, lse_stride,
+                        o_f32, o_f32_stride);
+}
+
+// One CTA per output row.  Inputs and the fp32 output are addressed by strides, so the same kernel
+// reads split partials ([row][split][D]), gathered per-rank partials ([rank][row][D]) and packed ones
+// ([rank][row][D + 1], LSE in the last column), and can write a packed row itself.
+// The parts are dealt to the warps, a lane taking every 32nd element of each (d_head 64: the second 64 of
+// the 128 accumulator slots stay empty); a thread that walks all parts of its element alone waits for one
+// pair of dependent loads after the other (B*H=8 Skv=131072, 148 splits, whole call: 93 us, now 85).
+constexpr int kCombineMaxWarps = 8;
+template <bool BF16>
+__global__ void __launch_bounds__(kCombineMaxWarps * 32)
+combine_kernel(const float* __restrict__ o_parts, const float* __restrict__ lse_parts,
+               int n_parts, long long part_stride_o, long long row_stride_o,
+               long long part_stride_l, long long row_stride_l, int d_head,
+               uint16_t* __restrict__ o, float* __restrict__ lse, long long lse_stride,
+               float* __restrict__ o_f32, long long o_f32_stride) {
+    __shared__ float part[kCombineMaxWarps][128], part_w[kCombineMaxWarps];
+    const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    const float* lp = lse_parts + (size_t)row * row_stride_l;
+    const float* op = o_parts + (size_t)row * row_stride_o + lane;
+    float m = -INFINITY;
+    for (int p = lane; p < n_parts; p += 32) m = fmaxf(m, lp[(size_t)p * part_stride_l]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    float wsum = 0.0f, a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (m > -INFINITY) {
+#pragma unroll 4
+        for (int p = warp; p < n_parts; p += n_warps) {
+            const float w = fast_ex2((lp[(size_t)p * part_stride_l] - m) * kLog2e);
+            wsum += w;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (i * 32 < d_head) a[i] = fmaf(w, op[(size_t)p * part_stride_o + i * 32], a[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) part[warp][i * 32 + lane] = a[i];
+    if (lane == 0) part_w[warp] = wsum;
+    __syncthreads();
+    float total = 0.0f;
+    for (int w = 0; w < n_warps; w++) total += part_w[w];
+    for (int d = threadIdx.x; d < d_head; d += blockDim.x) {
+        float acc = 0.0f;
+        for (int w = 0; w < n_warps; w++) acc += part[w][d];
+        write_row<BF16>(row, d, d_head, total > 0.0f ? acc / total : 0.0f, total > 0.0f ? m + kLn2 * log2f(total) : -INFINITY, o, lse,
+                        lse_stride, o_f32, o_f32_stride);
+    }
 }
 
 // A rank that holds no key of a KV-sequence-sharded cache contributes weight zero to the merge.
@@ -245,12 +355,14 @@ struct CombineOut {
 int launch_combine(const float* o_parts, const float* lse_parts, int n_parts, long long pso,
                    long long rso, long long psl, long long rsl, int rows, int d_head, const CombineOut& out,
                    int dtype, cudaStream_t stream) {
+    // two parts a warp, so that a warp's loads are in flight together and few warps idle
+    const int warps = n_parts >= 2 * kCombineMaxWarps ? kCombineMaxWarps : (n_parts + 1) / 2;
     if (dtype == FA_DTYPE_BF16)
-        combine_kernel<true><<<rows, d_head, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
+        combine_kernel<true><<<rows, warps * 32, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
                                                           static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
                                                           out.o_f32, out.o_f32_stride);
     else
-        combine_kernel<false><<<rows, d_head, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
+        combine_kernel<false><<<rows, warps * 32, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
                                                            static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
                                                            out.o_f32, out.o_f32_stride);
     FA_CUDA_TRY(cudaGetLastError());
@@ -298,21 +410,64 @@ void plan_splits(const fa_decode_args* a, int sm_count, int* splits_out, int* ke
     *keys_per_split_out = kps;
 }
 
-// The two launches of a decode step: per-split partials into `scratch` (fp32 O [bh][split][D], then,
+// CTAs per head of the one-launch path, 0 = take the two-launch path.  A head's splits must fit the portable
+// cluster size, and the whole grid the GPU at once (four CTAs of 8 warps an SM): a cluster keeps its
+// CTAs until the last has finished, so with more than one wave of them the two launches are as fast or
+// faster (f16 D=64 B*H=1024 Skv=4096, 4 splits: 180 against 159 us; bf16 D=128 B*H=128 Skv=4096, 8 splits: 49.3
+// against 47.9; bf16 D=64 B*H=128 Skv=2048, 4 splits, 512 CTAs: 14.4 against 15.2).  Heads that leave the GPU
+// empty get more CTAs than splits, up to two a SM and down to 64 keys each.
+int decode_cluster_ctas(long long bh, int splits, int seq_len_kv, int sm_count) {
+    if (splits > kMaxCluster || bh * splits > 4ll * sm_count) return 0;
+    long long n = 2ll * sm_count / bh;
+    const long long most = (seq_len_kv + 63) / 64;
+    if (n > most) n = most;
+    if (n < splits) n = splits;
+    return (int)(n > kMaxCluster ? kMaxCluster : n);
+}
+
+template <int D, bool BF16>
+int launch_decode_cluster(const fa_decode_args* a, int n_ctas, int sm_count, const CombineOut& out) {
+    const long long bh = (long long)a->batch_size * a->num_heads;
+    const int keys = (a->seq_len_kv + n_ctas - 1) / n_ctas;
+    // 16 warps where two such CTAs fit an SM and 8 warps would go round more than once
+    const bool wide = bh * n_ctas <= 2ll * sm_count && keys > kDecodeWarps * kUnroll * (256 / D);
+    auto kernel = wide ? decode_cluster_kernel<D, BF16, 2 * kDecodeWarps> : decode_cluster_kernel<D, BF16, kDecodeWarps>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(bh * n_ctas));
+    cfg.blockDim = dim3((wide ? 2 : 1) * kDecodeWarps * 32);
+    cfg.stream = static_cast<cudaStream_t>(a->stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)n_ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint16_t*>(a->q), static_cast<const uint16_t*>(a->k),
+                                   static_cast<const uint16_t*>(a->v), a->seq_len_kv, n_ctas, keys, a->scale * kLog2e,
+                                   static_cast<uint16_t*>(out.o), out.lse, out.lse_stride, out.o_f32, out.o_f32_stride));
+    return FA_OK;
+}
+
+// A decode step, in one launch or two: per-split partials into `scratch` (fp32 O [bh][split][D], then,
 // 256-byte aligned, LSE [bh][split]), and their merge into `out`.  Shared by fa_decode (caller's
 // workspace), fa_decode_static (the built-in array) and the KV-sharded entry (packed output).
-int decode_into(const fa_decode_args* a, int splits, int kps, void* scratch, const CombineOut& out) {
+int decode_into(const fa_decode_args* a, int splits, int kps, int sm_count, void* scratch, const CombineOut& out) {
     const long long bh = (long long)a->batch_size * a->num_heads;
     float* o_part = static_cast<float*>(scratch);
     float* lse_part = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) +
                                                align256((size_t)bh * splits * a->d_head * sizeof(float)));
+    const bool bf = a->dtype == FA_DTYPE_BF16;
+    if (const int n = decode_cluster_ctas(bh, splits, a->seq_len_kv, sm_count)) {
+        if (a->d_head == 128) return bf ? launch_decode_cluster<128, true>(a, n, sm_count, out) : launch_decode_cluster<128, false>(a, n, sm_count, out);
+        return bf ? launch_decode_cluster<64, true>(a, n, sm_count, out) : launch_decode_cluster<64, false>(a, n, sm_count, out);
+    }
     cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
     const unsigned grid = (unsigned)(bh * splits);
     const float sl2 = a->scale * kLog2e;
     const uint16_t* q = static_cast<const uint16_t*>(a->q);
     const uint16_t* k = static_cast<const uint16_t*>(a->k);
     const uint16_t* v = static_cast<const uint16_t*>(a->v);
-    const bool bf = a->dtype == FA_DTYPE_BF16;
 #define FA_LAUNCH_DECODE(DH, BF) \
     decode_partial_kernel<DH, BF><<<grid, kDecodeWarps * 32, 0, stream>>>(q, k, v, o_part, lse_part, \
         a->seq_len_kv, splits, kps, sl2)
@@ -359,7 +514,7 @@ FA_EXPORT int fa_decode(const fa_decode_args* a) {
     plan_splits(a, st->sm_count, &splits, &kps);
     const size_t need = fa_decode_workspace_bytes(a->batch_size, a->num_heads, a->d_head, splits);
     if (!a->workspace || a->workspace_bytes < need || !aligned16(a->workspace)) return FA_ERR_WORKSPACE;
-    return decode_into(a, splits, kps, a->workspace, caller_outputs(a));
+    return decode_into(a, splits, kps, st->sm_count, a->workspace, caller_outputs(a));
 }
 
 // ---------------------------------------------------------------------------
@@ -428,7 +583,7 @@ FA_EXPORT int fa_decode_static(const fa_decode_args* a) {
     if (fa_decode_workspace_bytes(a->batch_size, a->num_heads, a->d_head, splits) >
         (size_t)FA_DECODE_STATIC_SCRATCH_BYTES)
         return FA_ERR_WORKSPACE;
-    return decode_into(a, splits, kps, su->ptr, caller_outputs(a));
+    return decode_into(a, splits, kps, su->sm_count, su->ptr, caller_outputs(a));
 }
 
 // ---------------------------------------------------------------------------
@@ -703,7 +858,7 @@ FA_EXPORT int fa_decode_kv_sharded(const fa_decode_args* a, void* nccl_comm, flo
         CombineOut out;
         out.o_f32 = mine; out.o_f32_stride = a->d_head + 1;
         out.lse = mine + a->d_head; out.lse_stride = a->d_head + 1;
-        if ((rc = decode_into(a, splits, kps, a->workspace, out)) != FA_OK) return rc;
+        if ((rc = decode_into(a, splits, kps, st->sm_count, a->workspace, out)) != FA_OK) return rc;
     }
     // in place: the send buffer is this rank's block of the receive buffer
     r = api->all_gather(mine, gather, per_rank, ncclFloat, comm, stream);

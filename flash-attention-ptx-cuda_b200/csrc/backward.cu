@@ -111,8 +111,10 @@ __host__ __device__ constexpr uint32_t op16_col(int kk, bool in_place) {
 // delta = rowsum(dO o O).  d_head / 8 lanes per row, 16 bytes of each tensor per lane: a warp
 // covers 4 rows (d_head 64) or 2 (d_head 128) with one load instruction per tensor.
 template <bool BF16>
-__global__ void delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d_o,
-                             float* __restrict__ delta, long long n_rows, int d_head) {
+__global__ void delta_kernel(const uint16_t* o, const uint16_t* d_o,
+                             float* delta, long long n_rows, int d_head) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int lanes_per_row = d_head >> 3;                       // 8 or 16
     const int rows_per_warp = 32 / lanes_per_row;
     const int lane = threadIdx.x & 31;
@@ -178,8 +180,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUtensorMap ta1,
            const __grid_constant__ CUtensorMap tb0, const __grid_constant__ CUtensorMap tb1,
            const __grid_constant__ CUtensorMap to0, const __grid_constant__ CUtensorMap to1,
-           const float* __restrict__ lse, const float* __restrict__ delta, uint16_t* __restrict__ out0,
-           uint16_t* __restrict__ out1, int seq_len, int n_tiles, int n_bh, int n_items, float scale, int* status) {
+           const float* lse, const float* delta, uint16_t* out0,
+           uint16_t* out1, int seq_len, int n_tiles, int n_bh, int n_items, float scale, int* status) {
     using L = BwdSmem<D>;
     constexpr int NBOX = L::kNBox, kStages = L::kStages, NA = L::kNA;
     constexpr uint32_t FMT = BF16 ? kFmtBF16 : kFmtF16;
@@ -226,7 +228,6 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     const uint32_t b_s = base + NA * 2 * L::kTile;        // stationary buffers first, then the stages
     WaitCtl ctl{&abort_flag, status};
 
-    if (MODE == 0 && tid == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&bar_a[i]), 1); mbar_init(smem_u32(&bar_afree[i]), 2); }
         for (int i = 0; i < kStages; i++) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_acc[i]), NACC); }
@@ -247,6 +248,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    // The dK/dV kernel depends on `delta`.  Only after its wait does it let the dQ kernel start, so delta is
+    // complete for that one too, which reads nothing the dK/dV kernel writes and does not wait for it here.
+    if (MODE == 0) { grid_dependency_wait(); grid_launch_dependents(); }
     if (warp >= kComputeWarps) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdRegsRest));
 
     // gs: steps of the items this CTA has finished; a step's place in every ring is gs + t
@@ -602,7 +606,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     // outputs, so it never had to wait for it.  But whatever follows on the stream is ordered after
     // THIS kernel only: every thread waits here, after its own work, until the dK/dV grid has
     // completed and flushed, so that the end of this kernel implies the end of both.
-    if (MODE == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (MODE == 1) { grid_dependency_wait(); grid_launch_dependents(); }
     __syncthreads();
     if (warp == kTmemWarp) tmem_dealloc(tmem, 512);
 }
@@ -623,26 +627,14 @@ int launch_bwd(const fa_backward_args& a, DeviceState* st, const CUtensorMap& tq
     const long long n_items = n_bh * n_tiles;
     if (n_items > 0x7FFFFFFFll) return FA_ERR_INVALID_ARGUMENT;
     const long long grid = n_items < st->sm_count ? n_items : st->sm_count;   // persistent: one CTA per SM
-    // The dQ kernel (MODE 1) reads nothing the dK/dV kernel (MODE 0) writes, so it is launched as a
-    // programmatic dependent: its CTAs may start on SMs the first kernel no longer needs (that kernel
-    // signals at its start), instead of waiting for its last CTA.  delta comes from a kernel that
-    // completed before MODE 0 started.  Before it ends, every thread of the dQ kernel executes
-    // griddepcontrol.wait, so later work on the stream (or the next node of a captured graph) sees
-    // dK and dV complete as well.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kBwdThreads);
-    cfg.dynamicSmemBytes = L::kTotal;
-    cfg.stream = static_cast<cudaStream_t>(a.stream);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (MODE == 1) ? 1 : 0;
-    FA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, tdo, to0, to1, a.lse, delta, static_cast<uint16_t*>(out0),
-                                   static_cast<uint16_t*>(out1), a.seq_len, n_tiles, (int)n_bh, (int)n_items, a.scale,
-                                   st->status));
-    return FA_OK;
+    // delta, dK/dV and dQ kernel are each a programmatic dependent of the one before.  The dK/dV kernel (MODE
+    // 0) waits for delta; the dQ kernel (MODE 1) reads nothing that MODE 0 writes, so its CTAs start on the SMs
+    // MODE 0 no longer needs and work at once.  Before it ends, every thread of the dQ kernel executes
+    // griddepcontrol.wait, so later work on the stream (or the next node of a captured graph) sees dK and
+    // dV complete as well.
+    return launch_dependent(kernel, (unsigned)grid, kBwdThreads, L::kTotal, static_cast<cudaStream_t>(a.stream), 1, tq, tk, tv, tdo, to0,
+                            to1, a.lse, delta, static_cast<uint16_t*>(out0), static_cast<uint16_t*>(out1), a.seq_len, n_tiles, (int)n_bh,
+                            (int)n_items, a.scale, st->status);
 }
 
 // maps[0..3]: q, k, v, dO with boxes of 128 rows; maps[4..7]: the same with boxes of kW rows;
@@ -690,11 +682,9 @@ FA_EXPORT int fa_backward(const fa_backward_args* a) {
     {
         const long long rows_per_block = 8 * (32 / (a->d_head >> 3));      // 8 warps of 4 or 2 rows
         const unsigned blocks = (unsigned)((n_rows + rows_per_block - 1) / rows_per_block);
-        if (bf) delta_kernel<true><<<blocks, 256, 0, stream>>>(static_cast<const uint16_t*>(a->o),
-                    static_cast<const uint16_t*>(a->d_o), delta, n_rows, a->d_head);
-        else    delta_kernel<false><<<blocks, 256, 0, stream>>>(static_cast<const uint16_t*>(a->o),
-                    static_cast<const uint16_t*>(a->d_o), delta, n_rows, a->d_head);
-        FA_CUDA_TRY(cudaGetLastError());
+        const int drc = launch_dependent(bf ? delta_kernel<true> : delta_kernel<false>, blocks, 256, 0, stream, 1,
+                                         static_cast<const uint16_t*>(a->o), static_cast<const uint16_t*>(a->d_o), delta, n_rows, a->d_head);
+        if (drc != FA_OK) return drc;
     }
     CUtensorMap maps[11];
     const void* tensors[4] = {a->q, a->k, a->v, a->d_o};

@@ -34,6 +34,7 @@
 #include <mutex>
 
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace fa {
 namespace {
@@ -58,7 +59,7 @@ __device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
 
 __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
     uint4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                  : "l"(p));
     return r;
@@ -104,8 +105,8 @@ struct DecodeShared {
 
 // Keys [k_begin, k_end) of head bh, by the whole CTA; valid in threads < D.
 template <int D, bool BF16, int WARPS>
-__device__ __forceinline__ void decode_keys(DecodeShared<D, WARPS>& sm, const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
-                                            const uint16_t* __restrict__ v, int bh, int k_begin, int k_end, int seq_len_kv,
+__device__ __forceinline__ void decode_keys(DecodeShared<D, WARPS>& sm, const uint16_t* q, const uint16_t* k,
+                                            const uint16_t* v, int bh, int k_begin, int k_end, int seq_len_kv,
                                             float scale_log2, float& mm, float& ll, float& a) {
     constexpr int LPR = D / 8;           // lanes covering one row (8 elements = 16 bytes per lane)
     constexpr int RPW = 32 / LPR;        // rows per warp-wide load
@@ -116,7 +117,7 @@ __device__ __forceinline__ void decode_keys(DecodeShared<D, WARPS>& sm, const ui
 
     float qf[8];
     {
-        const uint4 qu = *reinterpret_cast<const uint4*>(q + (size_t)bh * D + dsl);
+        const uint4 qu = ld_stream_16(q + (size_t)bh * D + dsl);
         unpack8<BF16>(qu, qf);
 #pragma unroll
         for (int e = 0; e < 8; e++) qf[e] *= scale_log2;
@@ -207,11 +208,13 @@ __device__ __forceinline__ void decode_keys(DecodeShared<D, WARPS>& sm, const ui
 
 template <int D, bool BF16>
 __global__ void __launch_bounds__(kDecodeWarps * 32)
-decode_partial_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
-                      const uint16_t* __restrict__ v, float* __restrict__ o_part,
-                      float* __restrict__ lse_part, int seq_len_kv, int n_splits, int keys_per_split,
+decode_partial_kernel(const uint16_t* q, const uint16_t* k,
+                      const uint16_t* v, float* o_part,
+                      float* lse_part, int seq_len_kv, int n_splits, int keys_per_split,
                       float scale_log2) {
     __shared__ DecodeShared<D, kDecodeWarps> sm;
+    grid_dependency_wait();
+    grid_launch_dependents();
     // one-dimensional grid: the splits of a head are neighbours, and batch * heads is not limited to 65535
     const int bh = blockIdx.x / n_splits, split = blockIdx.x - bh * n_splits;
     const int k_begin = split * keys_per_split;
@@ -246,12 +249,14 @@ __device__ __forceinline__ void write_row(int row, int d, int d_head, float out,
 // 7.0 -> 4.5 us, f16 D=128 B*H=32 Skv=512 8.2 -> 3.9, Skv=4096 18.0 -> 16.5.
 template <int D, bool BF16, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-decode_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k, const uint16_t* __restrict__ v,
-                      int seq_len_kv, int n_ctas, int keys_per_cta, float scale_log2, uint16_t* __restrict__ o,
-                      float* __restrict__ lse, long long lse_stride, float* __restrict__ o_f32, long long o_f32_stride) {
+decode_cluster_kernel(const uint16_t* q, const uint16_t* k, const uint16_t* v,
+                      int seq_len_kv, int n_ctas, int keys_per_cta, float scale_log2, uint16_t* o,
+                      float* lse, long long lse_stride, float* o_f32, long long o_f32_stride) {
     __shared__ DecodeShared<D, WARPS> sm;
     __shared__ float res_a[D], res_m, res_l;
     const int bh = blockIdx.x / n_ctas, rank = blockIdx.x - bh * n_ctas;
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int k_begin = min(seq_len_kv, rank * keys_per_cta);
     float mm, ll, a;
     decode_keys<D, BF16, WARPS>(sm, q, k, v, bh, k_begin, min(seq_len_kv, k_begin + keys_per_cta), seq_len_kv, scale_log2, mm, ll, a);
@@ -299,13 +304,15 @@ decode_cluster_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict
 constexpr int kCombineMaxWarps = 8;
 template <bool BF16>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32)
-combine_kernel(const float* __restrict__ o_parts, const float* __restrict__ lse_parts,
+combine_kernel(const float* o_parts, const float* lse_parts,
                int n_parts, long long part_stride_o, long long row_stride_o,
                long long part_stride_l, long long row_stride_l, int d_head,
-               uint16_t* __restrict__ o, float* __restrict__ lse, long long lse_stride,
-               float* __restrict__ o_f32, long long o_f32_stride) {
+               uint16_t* o, float* lse, long long lse_stride,
+               float* o_f32, long long o_f32_stride) {
     __shared__ float part[kCombineMaxWarps][128], part_w[kCombineMaxWarps];
     const int row = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    grid_dependency_wait();
+    grid_launch_dependents();
     const float* lp = lse_parts + (size_t)row * row_stride_l;
     const float* op = o_parts + (size_t)row * row_stride_o + lane;
     float m = -INFINITY;
@@ -357,16 +364,9 @@ int launch_combine(const float* o_parts, const float* lse_parts, int n_parts, lo
                    int dtype, cudaStream_t stream) {
     // two parts a warp, so that a warp's loads are in flight together and few warps idle
     const int warps = n_parts >= 2 * kCombineMaxWarps ? kCombineMaxWarps : (n_parts + 1) / 2;
-    if (dtype == FA_DTYPE_BF16)
-        combine_kernel<true><<<rows, warps * 32, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
-                                                          static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
-                                                          out.o_f32, out.o_f32_stride);
-    else
-        combine_kernel<false><<<rows, warps * 32, 0, stream>>>(o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
-                                                           static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
-                                                           out.o_f32, out.o_f32_stride);
-    FA_CUDA_TRY(cudaGetLastError());
-    return FA_OK;
+    return launch_dependent(dtype == FA_DTYPE_BF16 ? combine_kernel<true> : combine_kernel<false>, rows, warps * 32, 0, stream, 1, o_parts,
+                            lse_parts, n_parts, pso, rso, psl, rsl, d_head, static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
+                            out.o_f32, out.o_f32_stride);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -432,21 +432,10 @@ int launch_decode_cluster(const fa_decode_args* a, int n_ctas, int sm_count, con
     // 16 warps where two such CTAs fit an SM and 8 warps would go round more than once
     const bool wide = bh * n_ctas <= 2ll * sm_count && keys > kDecodeWarps * kUnroll * (256 / D);
     auto kernel = wide ? decode_cluster_kernel<D, BF16, 2 * kDecodeWarps> : decode_cluster_kernel<D, BF16, kDecodeWarps>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(bh * n_ctas));
-    cfg.blockDim = dim3((wide ? 2 : 1) * kDecodeWarps * 32);
-    cfg.stream = static_cast<cudaStream_t>(a->stream);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)n_ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    FA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<const uint16_t*>(a->q), static_cast<const uint16_t*>(a->k),
-                                   static_cast<const uint16_t*>(a->v), a->seq_len_kv, n_ctas, keys, a->scale * kLog2e,
-                                   static_cast<uint16_t*>(out.o), out.lse, out.lse_stride, out.o_f32, out.o_f32_stride));
-    return FA_OK;
+    return launch_dependent(kernel, (unsigned)(bh * n_ctas), (wide ? 2 : 1) * kDecodeWarps * 32, 0, static_cast<cudaStream_t>(a->stream), n_ctas,
+                            static_cast<const uint16_t*>(a->q), static_cast<const uint16_t*>(a->k), static_cast<const uint16_t*>(a->v),
+                            a->seq_len_kv, n_ctas, keys, a->scale * kLog2e, static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
+                            out.o_f32, out.o_f32_stride);
 }
 
 // A decode step, in one launch or two: per-split partials into `scratch` (fp32 O [bh][split][D], then,
@@ -468,13 +457,10 @@ int decode_into(const fa_decode_args* a, int splits, int kps, int sm_count, void
     const uint16_t* q = static_cast<const uint16_t*>(a->q);
     const uint16_t* k = static_cast<const uint16_t*>(a->k);
     const uint16_t* v = static_cast<const uint16_t*>(a->v);
-#define FA_LAUNCH_DECODE(DH, BF) \
-    decode_partial_kernel<DH, BF><<<grid, kDecodeWarps * 32, 0, stream>>>(q, k, v, o_part, lse_part, \
-        a->seq_len_kv, splits, kps, sl2)
-    if (a->d_head == 128) { if (bf) FA_LAUNCH_DECODE(128, true); else FA_LAUNCH_DECODE(128, false); }
-    else                  { if (bf) FA_LAUNCH_DECODE(64, true);  else FA_LAUNCH_DECODE(64, false); }
-#undef FA_LAUNCH_DECODE
-    FA_CUDA_TRY(cudaGetLastError());
+    auto kernel = a->d_head == 128 ? (bf ? decode_partial_kernel<128, true> : decode_partial_kernel<128, false>)
+                                   : (bf ? decode_partial_kernel<64, true> : decode_partial_kernel<64, false>);
+    const int rc = launch_dependent(kernel, grid, kDecodeWarps * 32, 0, stream, 1, q, k, v, o_part, lse_part, a->seq_len_kv, splits, kps, sl2);
+    if (rc != FA_OK) return rc;
     // partials: o [bh][split][D], lse [bh][split]
     return launch_combine(o_part, lse_part, splits, a->d_head, (long long)splits * a->d_head, 1, splits,
                           (int)bh, a->d_head, out, a->dtype, stream);

@@ -54,6 +54,30 @@ int note_message(const char* msg, int code);
         if (fa_try_err_ != cudaSuccess) return ::fa::note_cuda_error(fa_try_err_, #expr); \
     } while (0)
 
+// Launches `kernel` as a programmatic dependent of whatever precedes it on the stream (cluster of
+// `cluster` CTAs): its launch and set-up overlap the end of that work.  The kernel must execute
+// grid_dependency_wait() before its first access to global memory.
+template <class... P, class... A>
+inline int launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, unsigned cluster,
+                            const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    FA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return FA_OK;
+}
+
 // Rank-3 tiled tensor map over a dense [n_heads, n_rows, row_elems] tensor with
 // 128-byte swizzle.  box_cols * elem_bytes must be 128; box_rows <= 256.
 // dtype is an FA_DTYPE_* value.

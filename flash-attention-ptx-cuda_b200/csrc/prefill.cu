@@ -168,7 +168,7 @@ __device__ __forceinline__ bool get_item(int k, int n_items, int n_bh, int n_qti
         it.hkv = it.bh - it.b * gq.n_hkv;
         it.tok0 = (gq.n_qt - 1 - qt_rev) * gq.tok_per_tile;
         it.t0 = it.split * gq.tiles_per_split;
-        it.kv_len = gq.seq_lens ? min(seq_len, max(0, __ldg(gq.seq_lens + it.b))) : seq_len;
+        it.kv_len = gq.seq_lens ? min(seq_len, max(0, gq.seq_lens[it.b])) : seq_len;
         // keys the tile's last token sees (the query tokens are the last n_tok entries of the cache)
         const int kv_vis = min(it.kv_len, it.kv_len - gq.n_tok + min(gq.n_tok, it.tok0 + gq.tok_per_tile));
         it.n_kv = min(gq.tiles_per_split, (max(kv_vis, 0) + kBN - 1) / kBN - it.t0);
@@ -224,9 +224,9 @@ template <int D, bool CAUSAL, bool BF16, bool FP8, bool GQA, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
-               float* __restrict__ lse_out, int seq_len, int n_bh, int n_qtiles, int n_items,
-               float scale_log2_in, const float* __restrict__ q_scale,
-               const float* __restrict__ k_scale, const float* __restrict__ v_scale, int* status,
+               float* lse_out, int seq_len, int n_bh, int n_qtiles, int n_items,
+               float scale_log2_in, const float* q_scale,
+               const float* k_scale, const float* v_scale, int* status,
                const GqaDev gq) {
     static_assert(!FP8 || (D == 128 && BF16), "e4m3 variant: d_head 128, bf16 output");
     static_assert(!GQA || !CAUSAL, "grouped-query decode: one query row per head, every key visible");
@@ -317,6 +317,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    // from here on global memory; the next kernel may take the SMs that run out of work
+    grid_dependency_wait();
+    grid_launch_dependents();
     const int n_rounds = (n_items + gridDim.x - 1) / gridDim.x;
 
     // Grouped-query decode: one 128-key tile of K or V of (batch, KV head) from the cache, issued by a whole
@@ -330,7 +333,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     auto cache_pages = [&](const Item& it, int j) -> int {
         const int off = lane << gq.page_shift, rr = (it.t0 + j) * kBN + off;
         if (off >= kBN || rr >= it.kv_len || j >= it.n_kv) return -1;
-        return __ldg(gq.block_table + static_cast<size_t>(it.b) * gq.table_stride + (rr >> gq.page_shift));
+        return gq.block_table[static_cast<size_t>(it.b) * gq.table_stride + (rr >> gq.page_shift)];
     };
     auto load_cache_tile = [&](uint32_t dst, uint32_t bytes, const CUtensorMap* tm, uint32_t bar, const Item& it, int j, int pages, auto paged) {
         constexpr int NB = FP8 ? 1 : NBOX;            // boxes per tile row: e4m3 rows are one 128-byte box
@@ -1087,11 +1090,9 @@ int launch_instance(const fa_prefill_args& a, DeviceState* st, const CUtensorMap
     order.by_heads = FastDiv(order.group);
     order.by_heads_last = FastDiv(n_bh % order.group ? n_bh % order.group : order.group);
     const unsigned grid = (unsigned)(n_items < st->sm_count ? n_items : st->sm_count);
-    kernel<<<grid, kThreads, L::kTotal, static_cast<cudaStream_t>(a.stream)>>>(
-        tq, tk, tv, to, a.lse, a.seq_len, n_bh, n_qtiles, (int)n_items, a.scale * kLog2e, a.q_scale,
-        a.k_scale, a.v_scale, st->status, order);
-    FA_CUDA_TRY(cudaGetLastError());
-    return FA_OK;
+    return launch_dependent(kernel, grid, kThreads, L::kTotal, static_cast<cudaStream_t>(a.stream), 1, tq, tk, tv, to, a.lse,
+                            a.seq_len, n_bh, n_qtiles, (int)n_items, a.scale * kLog2e, a.q_scale, a.k_scale, a.v_scale,
+                            st->status, order);
 }
 
 template <int D, bool BF16, bool FP8>
@@ -1123,10 +1124,8 @@ int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& 
                     g.n_tok, tok_per_tile, n_qt, tok_per_tile * g.group, walk,
                     FastDiv(g.n_splits), FastDiv((uint32_t)walk * n_qt), FastDiv(walk), FastDiv(last_heads), FastDiv(g.n_kv_heads), g.seq_lens, g.block_table, g.table_stride,
                     page_shift};
-    kernel<<<grid, kThreads, L::kTotal, g.stream>>>(tq, tk, tv, to, nullptr, g.kv_len, n_bh, 1, (int)n_items,
-                                                    g.scale * kLog2e, g.q_scale, g.k_scale, g.v_scale, st->status, gq);
-    FA_CUDA_TRY(cudaGetLastError());
-    return FA_OK;
+    return launch_dependent(kernel, grid, kThreads, L::kTotal, g.stream, 1, tq, tk, tv, to, nullptr, g.kv_len, n_bh, 1,
+                            (int)n_items, g.scale * kLog2e, g.q_scale, g.k_scale, g.v_scale, st->status, gq);
 }
 
 }  // namespace
@@ -1198,7 +1197,9 @@ int launch_decode_gqa(const GqaLaunch& g, DeviceState* st) {
 
 
 // e4m3 codes -> fp16 (exact), 16 codes per thread.
-__global__ void e4m3_to_f16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, long long n16) {
+__global__ void e4m3_to_f16_kernel(const uint4* src, uint4* dst, long long n16) {
+    grid_dependency_wait();
+    grid_launch_dependents();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n16) return;
     const uint4 c = src[i];
@@ -1260,9 +1261,8 @@ int launch_prefill_fp8(const fa_prefill_args& a, DeviceState* st) {
         c.k_scale = a.k_scale + h0;
         c.v_scale = a.v_scale + h0;
         const long long n16 = (long long)(nh * head_elems / 16);
-        e4m3_to_f16_kernel<<<(unsigned)((n16 + 255) / 256), 256, 0, stream>>>(static_cast<const uint4*>(c.v),
-                                                                            static_cast<uint4*>(v16), n16);
-        if (cudaGetLastError() != cudaSuccess) { rc = FA_ERR_CUDA; break; }
+        if ((rc = launch_dependent(e4m3_to_f16_kernel, (unsigned)((n16 + 255) / 256), 256, 0, stream, 1,
+                                   static_cast<const uint4*>(c.v), static_cast<uint4*>(v16), n16)) != FA_OK) break;
         CUtensorMap tq, tk, tv, to;
         if ((rc = make_tensor_map_3d(&tq, c.q, FA_DTYPE_E4M3, 128, a.seq_len, nh, 128, kBM)) != FA_OK) break;
         if ((rc = make_tensor_map_3d(&tk, c.k, FA_DTYPE_E4M3, 128, a.seq_len, nh, 128, kBN)) != FA_OK) break;

@@ -43,6 +43,16 @@ __device__ __forceinline__ bool elect_one() {
     return e != 0;
 }
 
+// Programmatic dependent launch (launch_dependent in host_common.h).  A kernel launched that way starts while
+// the kernel before it on the stream drains: everything it does before this wait may overlap that kernel,
+// every access to global memory comes after it (the wait ends when that kernel has completed and its
+// writes are visible; at once in a kernel launched without the attribute).  What the kernel before may have
+// written is read with plain loads: read-only ones (const __restrict__, __ldg, ld.global.nc) promise that
+// the data do not change while the kernel runs and may be moved above the wait.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start on the SMs this one leaves, once all its CTAs have got here.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------

@@ -32,8 +32,11 @@
 //     products(t) -> exponentials, dS -> accumulating MMAs(t)
 // run a step apart and fill each other's waits.  The 16-bit operands of the accumulating
 // MMAs get TMEM columns of their own, so a product buffer is free again as soon as its
-// values are in registers (d_head 128, MODE 0 has no columns left for that: there the
-// operands overwrite the products and the buffer is free when the accumulations are done).
+// values are in registers.  d_head 128, MODE 0 has no columns left for that: there the operands
+// overwrite the products, and a step runs as two chains, S^T -> P^T -> dV -> next S^T and dP^T -> dS^T
+// -> dK -> next dP^T, each with barriers of its own, so that one half's tensor work overlaps the
+// other's arithmetic (as one chain, with the parity's warps meeting once a step, bf16 causal B*H=32
+// S=4096 took 472 us instead of 428 and f16 B*H=24 S=2048 without a mask 193 instead of 166).
 //   warps 0-7    even steps, two threads per stationary row (TMEM lane): warps 0-3 take the
 //                first 32 streamed columns of a step, warps 4-7 the other 32: exponentials,
 //                dS, 16-bit operands to TMEM; at the end of an item conversion of the
@@ -207,18 +210,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
     //   bar_full[s] / bar_acc[s]  streamed tiles of stage s loaded / the accumulations that read them done
     //   bar_t[g] / bar_tfree[g]   products of parity g done / their values are in registers
     //   bar_p[g]                  16-bit operands of parity g in TMEM
+    //   bar_t1, bar_p1, bar_acc1  in place: the same for the dP^T / dS^T / dK half of a step, bar_t, bar_p and
+    //                             bar_acc then stand for its S^T / P^T / dV half
     //   bar_done / bar_accfree    an item's accumulators complete / read out
     //   bar_ostaged / bar_ofree[b] an item's output tiles staged in buffer b / read by their TMA store
     __shared__ __align__(8) uint64_t bar_a[2], bar_afree[2], bar_full[kStages], bar_acc[kStages], bar_t[2], bar_tfree[2],
-        bar_p[2], bar_done, bar_accfree, bar_ostaged, bar_ofree[2];
+        bar_p[2], bar_acc1[INPLACE ? kStages : 1], bar_t1[2], bar_p1[2], bar_done, bar_accfree, bar_ostaged, bar_ofree[2];
     // MODE 0: statistics of the streamed queries of the current / next step, per column pair
     // {-lse*log2e (col 0, col 1), -delta*scale (col 0, col 1)}: the addends of the two packed FMAs.
-    // WARP_STATS: every compute warp stages the 32 columns it works on itself (lane j: column j), so
-    // a __syncwarp orders writes and reads and the warps of a parity need not meet.  Otherwise
-    // (d_head 128, where that measured 9 % slower) threads 0..63 of a parity stage its 64 columns
-    // and the parity's eight warps meet at a named barrier once per step.
-    constexpr bool WARP_STATS = !INPLACE;
-    __shared__ __align__(16) float st_neg[MODE != 0 ? 1 : (WARP_STATS ? kComputeWarps : 2)][2][WARP_STATS ? 16 : 32][4];
+    // Every compute warp stages the 32 columns it works on itself (lane j: column j), so a __syncwarp
+    // orders writes and reads and the warps of a parity need not meet.
+    __shared__ __align__(16) float st_neg[MODE != 0 ? 1 : kComputeWarps][2][16][4];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -230,11 +232,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) { mbar_init(smem_u32(&bar_a[i]), 1); mbar_init(smem_u32(&bar_afree[i]), 2); }
-        for (int i = 0; i < kStages; i++) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_acc[i]), NACC); }
+        for (int i = 0; i < kStages; i++) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_acc[i]), INPLACE ? 1 : NACC); }
+        if (INPLACE)
+            for (int i = 0; i < kStages; i++) mbar_init(smem_u32(&bar_acc1[i]), 1);
         for (int i = 0; i < 2; i++) {
             mbar_init(smem_u32(&bar_t[i]), 1);
             mbar_init(smem_u32(&bar_tfree[i]), 8);       // one arrival per compute warp of the parity
             mbar_init(smem_u32(&bar_p[i]), 8);
+            mbar_init(smem_u32(&bar_t1[i]), 1);
+            mbar_init(smem_u32(&bar_p1[i]), 8);
         }
         mbar_init(smem_u32(&bar_done), NACC);
         mbar_init(smem_u32(&bar_accfree), kComputeWarps);
@@ -276,7 +282,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
             for (int t = 0; t < it.n_steps; t++) {
                 const int T = gs + t, s = T % kStages;
                 // the stage held step T - kStages: its accumulations must have completed
-                if (T >= kStages && !mbar_wait(smem_u32(&bar_acc[s]), ((T - kStages) / kStages) & 1, ctl, kBwdBarFree)) { ok = false; break; }
+                if (T >= kStages) {
+                    ok = mbar_wait(smem_u32(&bar_acc[s]), ((T - kStages) / kStages) & 1, ctl, kBwdBarFree);
+                    if (INPLACE) ok = ok && mbar_wait(smem_u32(&bar_acc1[s]), ((T - kStages) / kStages) & 1, ctl, kBwdBarFree);
+                    if (!ok) break;
+                }
                 const uint32_t dst = b_s + s * 2 * L::kTileB;
                 if (elect_one()) {
                     mbar_arrive_expect_tx(smem_u32(&bar_full[s]), 2 * L::kTileB);
@@ -321,12 +331,21 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
                         mma_f16_ss(tb, da0 + offa, db0 + offb, idesc_t, kk > 0);
                     }
+                    if (INPLACE) tc_commit(smem_u32(&bar_t[g]));
+                }
+                if (INPLACE) {
+                    __syncwarp();
+                    // the dP^T half has a chain of its own: dK of step T - 2, not dV, must be done
+                    if (T >= 2 && !mbar_wait(smem_u32(&bar_acc1[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc)) { ok = false; break; }
+                    tc_fence_after();
+                }
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
                         mma_f16_ss(tb + kW, da1 + offa, db1 + offb, idesc_t, kk > 0);
                     }
-                    tc_commit(smem_u32(&bar_t[g]));
+                    tc_commit(smem_u32(INPLACE ? &bar_t1[g] : &bar_t[g]));
                 }
                 __syncwarp();
                 issued = true;
@@ -356,7 +375,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
         for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
             for (int t = 0; t < it.n_steps; t++) {
                 const int T = gs + t, s = T % kStages, g = T & 1;
-                if (!mbar_wait(smem_u32(&bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP)) { ok = false; break; }
+                if (!mbar_wait(smem_u32(INPLACE && x == 1 ? &bar_p1[g] : &bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP)) { ok = false; break; }
                 // the accumulators of the item before must have been read out
                 if (t == 0 && k >= 1 && !mbar_wait(smem_u32(&bar_accfree), (k - 1) & 1, ctl, kBwdBarFree)) { ok = false; break; }
                 tc_fence_after();
@@ -366,7 +385,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
 #pragma unroll
                     for (int kk = 0; kk < kW / 16; kk++)
                         mma_f16_ts(acc, op + op16_col(kk, INPLACE), db + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
-                    tc_commit(smem_u32(&bar_acc[s]));
+                    tc_commit(smem_u32(INPLACE && x == 1 ? &bar_acc1[s] : &bar_acc[s]));
                     if (t == it.n_steps - 1) tc_commit(smem_u32(&bar_done));
                 }
                 __syncwarp();
@@ -396,12 +415,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdRegsCompute));
         const int g = warp >> 3;                            // parity of the steps this warp works on
         const int half = (warp >> 2) & 1;                   // which 32 streamed columns of a step
-        const int gt = tid & 255;                           // thread within the parity's warps
-        // MODE 0: the streamed column of a step whose statistics this thread stages, and where
-        const int st_col = WARP_STATS ? half * 32 + lane : gt;
-        const bool st_mine = WARP_STATS || gt < kW;
-        const int st_set = (MODE != 0) ? 0 : (WARP_STATS ? warp : g);
-        const int st_pair = WARP_STATS ? (lane >> 1) : (gt >> 1) & 31, st_pair0 = WARP_STATS ? 0 : half * 16;
+        const int st_col = half * 32 + lane;                // MODE 0: the streamed column of a step whose statistics this thread stages
         const int r = tid & (kT - 1);                       // == TMEM lane
         const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const float scale_log2 = scale * kLog2e;
@@ -414,7 +428,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
         auto prefetch = [&](const BwdItem& x, int gs_x, int ahead, float& l2, float& dl) {
             const int t = ((g ^ gs_x) & 1) + 2 * ahead;
             const int row = (MODE == 1) ? x.tile * kT + r : x.row0 + t * kW + st_col;
-            const bool mine = (MODE == 1) ? (ahead == 0) : (st_mine && t < x.n_steps);
+            const bool mine = (MODE == 1) ? (ahead == 0) : t < x.n_steps;
             l2 = INFINITY;
             dl = 0.0f;
             if (mine && row < seq_len) {
@@ -437,19 +451,22 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
             const float* lse_h = lse + static_cast<size_t>(it.bh) * seq_len;
             const float* delta_h = delta + static_cast<size_t>(it.bh) * seq_len;
             const float row_lse2 = pf_l2, row_delta = pf_dl;    // MODE 1
-            // MODE 0: statistics of the streamed queries, one per column: threads 0..kW-1 of the parity
-            // fetch those of its step after next from global memory and stage those of its next step in
-            // shared memory while the current ones are in use; rows past the end get LSE = +inf
+            // MODE 0: statistics of the streamed queries, one per column: a thread fetches that of its
+            // parity's step after next from global memory and stages that of its next step in shared
+            // memory while the current ones are in use; rows past the end get LSE = +inf
             auto fetch_stats = [&](int t, float& l2, float& dl) {
                 const int qi = row0 + t * kW + st_col;
                 l2 = INFINITY;
                 dl = 0.0f;
-                if (MODE == 0 && st_mine && t < n_steps && qi < seq_len) { l2 = lse_h[qi] * kLog2e; dl = delta_h[qi]; }
+                if (MODE == 0 && t < n_steps && qi < seq_len) { l2 = lse_h[qi] * kLog2e; dl = delta_h[qi]; }
             };
+            // D 64: {-lse (2 columns), -delta (2 columns)} per column pair, one load for both uses; in place, where
+            // they are used one after the other: -lse of all 32 columns, then -delta
             auto stage_stats = [&](int slot, float l2, float dl) {
-                if (st_mine) {
-                    st_neg[st_set][slot][st_pair][st_col & 1] = -l2;
-                    st_neg[st_set][slot][st_pair][2 + (st_col & 1)] = -dl * scale;
+                if constexpr (MODE == 0) {
+                    float* st = &st_neg[warp][slot][0][0];
+                    st[INPLACE ? lane : (lane >> 1) * 4 + (lane & 1)] = -l2;
+                    st[INPLACE ? 32 + lane : (lane >> 1) * 4 + 2 + (lane & 1)] = -dl * scale;
                 }
             };
             const int t_first = (g ^ gs) & 1;               // this parity's first step of the item
@@ -466,18 +483,12 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 const int c0 = row0 + t * kW;               // first streamed row (= column of T0/T1) of the step
                 const uint32_t tb = tmem + lane_off + g * 128 + half * 32;
                 ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_t[g]), i & 1, ctl, kBwdBarT));
-                if (MODE == 0 && !WARP_STATS) {
-                    // the parity's warps are past their reads of the other slot; this step's values
-                    // (written a step ago) become visible; all eight warps leave together on an abort
-                    if (group_sync_or(1 + g, 256, !ok)) { ok = false; break; }
-                } else if (!ok) {
-                    break;
-                }
+                if (!ok) break;
                 if (MODE == 0) {
                     stage_stats((i + 1) & 1, nx_l2, nx_dl);
-                    // own staging: every lane is past its reads of that slot (the warp has synchronised
-                    // since), and this step's values, written a step ago, are visible from here
-                    if (WARP_STATS) __syncwarp();
+                    // every lane is past its reads of that slot (the warp has synchronised since), and this
+                    // step's values, written a step ago, are visible from here
+                    __syncwarp();
                     fetch_stats(t + 4, nx_l2, nx_dl);
                 }
                 tc_fence_after();
@@ -486,11 +497,64 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 const bool need_mask = (MODE == 0) ? (CAUSAL && c0 < (tile + 1) * kT)
                                                    : ((CAUSAL && c0 + kW > tile * kT) || c0 + kW > seq_len);
                 uint32_t pk[16], dk[16];
+                if constexpr (INPLACE) {
+                    // The operands overwrite the products they come from, so a step's two halves run as two
+                    // chains: S^T -> P^T -> dV and dP^T -> dS^T -> dK.  P^T goes to the tensor core before dP^T is
+                    // looked at, and the next S^T of this parity waits for that dV only.
+                    const float* st = &st_neg[warp][i & 1][0][0];
+                    uint32_t sv[32];
+                    tmem_ld32_wait(tb, sv);
+                    if (need_mask) {
+#pragma unroll
+                        for (int e = 0; e < 32; e++) sv[e] = r_glob <= c0 + half * 32 + e ? sv[e] : 0xff800000u;   // -inf
+                    }
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4) {
+                        const float4 l4 = *reinterpret_cast<const float4*>(st + e);
+                        const uint64_t xa = fma2(pack2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale_log2_2, pack2(l4.x, l4.y));
+                        const uint64_t xb = fma2(pack2(__uint_as_float(sv[e + 2]), __uint_as_float(sv[e + 3])), scale_log2_2, pack2(l4.z, l4.w));
+                        float x0, x1, x2, x3;
+                        unpack2(xa, x0, x1);
+                        unpack2(xb, x2, x3);
+                        const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
+                        sv[e] = __float_as_uint(p0); sv[e + 1] = __float_as_uint(p1);
+                        sv[e + 2] = __float_as_uint(p2); sv[e + 3] = __float_as_uint(p3);
+                        pk[e >> 1] = pack_16<BF16>(p0, p1);
+                        pk[(e >> 1) + 1] = pack_16<BF16>(p2, p3);
+                    }
+                    tmem_st_x16(tmem + lane_off + OPP0 + g * OP_STRIDE + half * 32u, pk);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_p[g]));
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_t1[g]), i & 1, ctl, kBwdBarT));
+                    if (!ok) break;
+                    tc_fence_after();
+                    uint32_t dv[32];
+                    tmem_ld32_wait(tb + kW, dv);
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(st + 32 + e);
+                        const uint64_t ga = fma2(pack2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), scale2, pack2(d4.x, d4.y));
+                        const uint64_t gb = fma2(pack2(__uint_as_float(dv[e + 2]), __uint_as_float(dv[e + 3])), scale2, pack2(d4.z, d4.w));
+                        float e0, e1;
+                        unpack2(mul2(pack2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), ga), e0, e1);
+                        dk[e >> 1] = pack_16<BF16>(e0, e1);
+                        unpack2(mul2(pack2(__uint_as_float(sv[e + 2]), __uint_as_float(sv[e + 3])), gb), e0, e1);
+                        dk[(e >> 1) + 1] = pack_16<BF16>(e0, e1);
+                    }
+                    tmem_st_x16(tmem + lane_off + OPD0 + g * OP_STRIDE + half * 32u, dk);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_p1[g]));
+                    continue;
+                }
 #pragma unroll
                 for (int c = 0; c < 2; c++) {               // 16 columns of each product at a time
                     uint32_t sv[16], dv[16];
                     tmem_ld16x2_wait(tb + c * 16, sv, tb + kW + c * 16, dv);
-                    if (c == 1 && !INPLACE) {
+                    if (c == 1) {
                         // the product buffer is free for this parity's next step
                         tc_fence_before();
                         __syncwarp();
@@ -508,7 +572,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     for (int e = 0; e < 16; e += 2) {
                         uint64_t neg_l2 = row_neg_l2, neg_dl = row_neg_dl;
                         if (MODE == 0) {                    // per column: one 16-byte shared load per pair
-                            const float4 st = *reinterpret_cast<const float4*>(st_neg[st_set][i & 1][st_pair0 + c * 8 + (e >> 1)]);
+                            const float4 st = *reinterpret_cast<const float4*>(st_neg[MODE == 0 ? warp : 0][i & 1][c * 8 + (e >> 1)]);
                             neg_l2 = pack2(st.x, st.y);
                             neg_dl = pack2(st.z, st.w);
                         }
@@ -524,17 +588,12 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                         dk[c * 8 + (e >> 1)] = pack_16<BF16>(e0, e1);
                     }
                 }
-                if (!INPLACE && T >= 2) {
-                    // the operand columns of this parity were read by the accumulations of step T-2
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc))) {
-                        ok = false;
-                        if (MODE == 0 && !WARP_STATS) continue;   // leave with the others at the next rendezvous
-                        break;
-                    }
+                // the operand columns of this parity were read by the accumulations of step T-2
+                if (T >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc))) {
+                    ok = false;
+                    break;
                 }
-                // each half writes its 16 columns of pairs; in place they land on the first half of the
-                // 32 columns this thread has read itself
-                const uint32_t op_off = INPLACE ? half * 32u : half * 16u;
+                const uint32_t op_off = half * 16u;         // each half writes its 16 columns of pairs
                 if (MODE == 0) tmem_st_x16(tmem + lane_off + OPP0 + g * OP_STRIDE + op_off, pk);
                 tmem_st_x16(tmem + lane_off + OPD0 + g * OP_STRIDE + op_off, dk);
                 tmem_wait_st();
@@ -542,7 +601,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bar_p[g]));
             }
-            if (!ok && (MODE == 1 || WARP_STATS)) break;
+            if (!ok) break;
             BwdItem nx;
             const bool have_nx = bwd_item<CAUSAL, MODE>(k + 1, n_items, n_bh, n_tiles, seq_len, nx);
             if (have_nx) {

@@ -869,6 +869,171 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int r_in_tile = (warp & 3) * 32 + lane;     // 0..127 == TMEM lane; one thread owns the whole row
         const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t t_o = tmem + lane_off + O_COL + (SPLIT ? grp * D : 0);
+        if (GQA && gq.live_rows <= 16) {
+            // Decode with at most 16 live rows.  As below only the first warp of each group has work, but it
+            // takes its rows through the 16-lane TMEM shapes, which spread a row over four threads: 32 exponentials
+            // a thread and tile (64 with more than 8 rows) instead of 128.  Both groups' working warps share one
+            // scheduler, and 256 exponentials per pair of tiles on its MUFU were the longest stage of decode over
+            // an e4m3 cache (B=32 Hkv=8 Skv=16384, 4 heads a group: 210 -> 198 us; bf16 B=1 Skv=4096 11.9 -> 11.0).
+            const bool idle = (warp & 3) != 0;
+            const int quad = lane & 3, row0 = lane >> 2;  // this thread: rows row0 and row0 + 8
+            const bool two = gq.live_rows > 8;
+            int g0 = 0, it_n = 0;
+            bool ok = true;
+            for (int r = 0; ok && r < n_rounds; r++) {
+                Item it;
+                if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
+                const int lim0 = it.kv_len - gq.n_tok + 1 + it.tok0;           // keys the tile's first token sees
+                const int limit0 = min(it.kv_len, lim0 + row0 / gq.group), limit1 = min(it.kv_len, lim0 + (row0 + 8) / gq.group);
+                float scale_log2 = scale_log2_in;
+                if constexpr (FP8) scale_log2 *= q_scale[it.bh] * k_scale[it.bh];
+                const uint64_t scale2 = pack2(scale_log2, scale_log2);
+                float m0 = -1e30f, m1 = -1e30f;           // reference max of this thread's partial sums
+                uint64_t sum0 = pack2(0.0f, 0.0f), sum1 = sum0;
+                for (int j = (g0 & 1) == grp ? 0 : 1; j < it.n_kv; j += 2) {
+                    const int g = g0 + j, u = g % kNU;
+                    const int kv_start = (it.t0 + j) * kBN;
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, kBarSFull))) { ok = false; break; }
+                    tc_fence_after();
+                    if (idle) {
+                        tc_fence_before();
+                        if (lane == 0) mbar_arrive(smem_u32(&bar_pf[u]));
+                        continue;
+                    }
+                    const uint32_t t_s = tmem + lane_off + u * 128;
+                    uint32_t s[64];
+                    tmem_ld_16x128cols_wait(t_s, s);
+                    if (min(it.kv_len, lim0) - kv_start < kBN) {               // tile touches the mask or the ragged end
+#pragma unroll
+                        for (int i = 0; i < 16; i++)
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                const int col = kv_start + 8 * i + 2 * quad + e;
+                                if (col >= limit0) s[4 * i + e] = 0xff800000u;           // -inf
+                                if (col >= limit1) s[4 * i + 2 + e] = 0xff800000u;
+                            }
+                    }
+                    float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        x0 = max3(x0, __uint_as_float(s[4 * i]), __uint_as_float(s[4 * i + 1]));
+                        x1 = max3(x1, __uint_as_float(s[4 * i + 2]), __uint_as_float(s[4 * i + 3]));
+                    }
+#pragma unroll
+                    for (int off = 1; off < 4; off <<= 1) {
+                        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
+                        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
+                    }
+                    // finite, so that a row without a visible key gets p = 0
+                    float n0 = fmaxf(x0 * scale_log2, -1e30f), n1 = fmaxf(x1 * scale_log2, -1e30f);
+                    float f0 = 1.0f, f1 = 1.0f;           // factors for what O holds
+                    bool changed = false;
+                    const uint32_t slot0 = smem_u32(&m_slot[it_n & 1][row0]), slot1 = slot0 + 8 * sizeof(uint2);
+                    if (j > 0) {
+                        uint32_t b0 = 0, b1 = 0, tag0 = 0, tag1 = 0;
+                        const int w = bounded_wait(
+                            [&] {
+                                asm volatile("ld.volatile.shared.v2.b32 {%0, %1}, [%2];" : "=r"(b0), "=r"(tag0) : "r"(slot0));
+                                asm volatile("ld.volatile.shared.v2.b32 {%0, %1}, [%2];" : "=r"(b1), "=r"(tag1) : "r"(slot1));
+                                return tag0 == static_cast<uint32_t>(g - 1) && tag1 == static_cast<uint32_t>(g - 1);
+                            },
+                            [&] { return *ctl.abort_flag != 0; }, [] { return global_timer_ns(); }, kWaitLimitNs, 256u);
+                        if (!__all_sync(0xffffffffu, w == kWaitDone)) {
+                            if (w == kWaitTimedOut) {
+                                *ctl.abort_flag = 1;
+                                atomicCAS(ctl.status, 0, wait_timeout_word(kBarM));
+                            }
+                            ok = false;
+                            break;
+                        }
+                        const float p0 = __uint_as_float(b0), p1 = __uint_as_float(b1);
+                        const bool c0 = n0 > p0 + kRescaleThreshold, c1 = n1 > p1 + kRescaleThreshold;
+                        n0 = c0 ? n0 : p0;
+                        n1 = c1 ? n1 : p1;
+                        f0 = c0 ? ex2_approx(p0 - n0) : 1.0f;
+                        f1 = c1 ? ex2_approx(p1 - n1) : 1.0f;
+                        changed = c0 || c1;
+                    }
+                    if (quad == 0) {
+                        asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(slot0), "r"(__float_as_uint(n0)), "r"(static_cast<uint32_t>(g)) : "memory");
+                        asm volatile("st.volatile.shared.v2.b32 [%0], {%1, %2};" ::"r"(slot1), "r"(__float_as_uint(n1)), "r"(static_cast<uint32_t>(g)) : "memory");
+                    }
+                    const float k0 = ex2_approx(m0 - n0), k1 = ex2_approx(m1 - n1);
+                    sum0 = mul2(sum0, pack2(k0, k0));
+                    sum1 = mul2(sum1, pack2(k1, k1));
+                    m0 = n0;
+                    m1 = n1;
+                    if (__any_sync(0xffffffffu, changed)) {       // rare: rescale O before this tile's P V
+                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, kBarPV))) { ok = false; break; }
+                        tc_fence_after();
+                        const float r0 = __shfl_sync(0xffffffffu, f0, (lane & 7) * 4), r1 = __shfl_sync(0xffffffffu, f1, (lane & 7) * 4);
+                        const float factor = lane < 8 ? r0 : lane < 16 ? r1 : 1.0f;   // of TMEM lane `lane`
+#pragma unroll 1
+                        for (int c = 0; c < D / 32; c++) {
+                            uint32_t t[32];
+                            tmem_ld32_wait(t_o + c * 32, t);
+#pragma unroll
+                            for (int i = 0; i < 32; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * factor);
+                            tmem_st_x32(t_o + c * 32, t);
+                        }
+                        tmem_wait_st();
+                    }
+                    uint32_t pk[32];
+                    const uint64_t neg0 = pack2(-n0, -n0), neg1 = pack2(-n1, -n1);
+                    auto row_p = [&](int first, uint64_t neg, uint64_t& sum, int out) {
+                        uint64_t acc = pack2(0.0f, 0.0f);
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            float t0, t1;
+                            unpack2(fma2(pack2(__uint_as_float(s[4 * i + first]), __uint_as_float(s[4 * i + first + 1])), scale2, neg), t0, t1);
+                            const float p0 = ex2_approx(t0), p1 = ex2_approx(t1);
+                            if (i & 1) acc = add2(acc, pack2(p0, p1));
+                            else       sum = add2(sum, pack2(p0, p1));
+                            pk[2 * i + out] = pack_16<P_BF16>(p0, p1);
+                        }
+                        sum = add2(sum, acc);
+                    };
+                    row_p(0, neg0, sum0, 0);
+                    if (two) {
+                        row_p(2, neg1, sum1, 1);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) pk[2 * i + 1] = 0u;
+                    }
+                    tmem_st_16x64cols(t_s, pk);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_pf[u]));
+                }
+                if (!ok) break;
+                const int par = it_n & 1;
+                if (it_n >= 2 &&
+                    !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, kBarStatsFree))) { ok = false; break; }
+                if (!idle) {
+                    float a, b, c, d;
+                    unpack2(sum0, a, b);
+                    unpack2(sum1, c, d);
+                    a += b;
+                    c += d;
+#pragma unroll
+                    for (int off = 1; off < 4; off <<= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, off);
+                        c += __shfl_xor_sync(0xffffffffu, c, off);
+                    }
+                    if (quad == 0) {
+                        xm[par][grp][row0] = m0;
+                        xsum[par][grp][row0] = a;
+                        xm[par][grp][row0 + 8] = m1;
+                        xsum[par][grp][row0 + 8] = c;
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bar_stats[par]));
+                g0 += it.n_kv;
+                it_n++;
+            }
+        } else {
         int g0 = 0, it_n = 0;
         bool ok = true;
 
@@ -1046,6 +1211,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             g0 += it.n_kv;
             it_n++;
+        }
         }
     }
 

@@ -76,7 +76,6 @@ constexpr int kRegsHelper = 64;          // warps 12-15
 static_assert(256 * kRegsSoftmax + 128 * kRegsOther + 128 * kRegsHelper <= kThreads * kRegsLaunch,
               "setmaxnreg targets exceed the CTA's register pool");
 constexpr int kNU = 3;                   // score buffers in TMEM (S, then P in place), used round-robin
-constexpr int kRing = 4;                 // entries of the Q K^T / P V completion rings
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;   // log2 units: rescale only if max grew > 2^8
@@ -97,7 +96,7 @@ __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint16_t v) {
 }
 
 
-template <int D, bool FP8, bool V8 = FP8>
+template <int D, bool FP8, bool V8 = FP8, bool SMALL = false>
 struct PrefillSmem {
     static constexpr int kNBox    = D / 64;               // 64-column (128-byte) boxes per 16-bit row
     static constexpr int kBox     = 128 * 128;            // one box: 128 rows x 128 bytes
@@ -106,13 +105,14 @@ struct PrefillSmem {
     static constexpr int kKBytes  = kQBytes;
     static constexpr int kVBytes  = kNBox * kBox;         // 16-bit V operand of P V (e4m3: converted copy)
     static constexpr int kV8Bytes = V8 ? kBox : 0;       // landing buffers of the e4m3 V tiles
-    static constexpr int kOBytes  = kNBox * kBox;         // epilogue staging (16-bit output tile)
+    static constexpr int kOBytes  = SMALL ? 0 : kNBox * kBox;   // epilogue staging (16-bit output tile)
     // V8 (decode over an e4m3 cache): three landing buffers of K and V and two converted (fp16) V tiles; the bytes in
     // flight are what the cache's bandwidth needs (2, 2 and 3, the same shared memory: 198 us instead of 181,
-    // B=32 Hkv=8 Skv=16384).
-    static constexpr int NK  = (D == 64) ? 4 : (V8 ? 3 : 2);
-    static constexpr int NV  = (D == 64) ? 4 : 2;
-    static constexpr int NV8 = V8 ? 3 : 0;
+    // B=32 Hkv=8 Skv=16384).  SMALL has no output to stage and takes the room for loads in flight as well: with
+    // two stages a lone CTA waits for a load's latency every other tile (see `ahead` at the launch).
+    static constexpr int NK  = (D == 64) ? (SMALL ? 6 : 4) : V8 ? (SMALL ? 4 : 3) : (SMALL ? 3 : 2);
+    static constexpr int NV  = (D == 64) ? (SMALL ? 6 : 4) : V8 ? 2 : (SMALL ? 3 : 2);
+    static constexpr int NV8 = V8 ? (SMALL ? 4 : 3) : 0;
     static constexpr int kTotal = kQBytes + NK * kKBytes + NV * kVBytes + NV8 * kV8Bytes + kOBytes + 1024;
 };
 
@@ -134,6 +134,7 @@ struct GqaDev {
     const int* block_table; // paged cache: [batch][table_stride] page numbers, or null
     int table_stride;
     int page_shift;         // log2(page size)
+    int ahead;              // SMALL: key tiles loaded ahead, at most the stage counts
 };
 
 // Work list: item index -> (query tile, head), heaviest first when causal.  In grouped-query
@@ -223,7 +224,8 @@ __device__ __forceinline__ bool get_item(int k, int n_items, int n_bh, int n_qti
 // their own and warps 12-15 convert each one in shared memory (V8).
 // The Q and K scales fold into the softmax scale, the V scale into the final normalisation;
 // the output is bf16.
-template <int D, bool CAUSAL, bool BF16, bool FP8, bool GQA, bool GROUPED>
+// SMALL (grouped-query decode): at most 16 live rows in a query tile.
+template <int D, bool CAUSAL, bool BF16, bool FP8, bool GQA, bool GROUPED, bool SMALL>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -234,7 +236,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     static_assert(!FP8 || (D == 128 && BF16), "e4m3 variant: d_head 128, bf16 output");
     static_assert(!GQA || !CAUSAL, "grouped-query decode: one query row per head, every key visible");
     constexpr bool V8 = FP8 && GQA;                       // V arrives as e4m3 and is converted in shared memory
-    using L = PrefillSmem<D, FP8, V8>;
+    using L = PrefillSmem<D, FP8, V8, SMALL>;
+    static_assert(!SMALL || GQA, "few rows: decode only");
+    constexpr int ROWS = SMALL ? 16 : 128;                // rows with statistics
+    constexpr int kRing = (D == 64 && SMALL) ? 8 : 4;     // entries of the Q K^T / P V completion rings
     constexpr int NBOX = L::kNBox, NK = L::NK, NV = L::NV;
     constexpr uint32_t O_COL = kNU * 128;
     // d_head 64 leaves TMEM for an accumulator of O per softmax group.  Each group then works on its
@@ -264,9 +269,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     __shared__ __align__(8) uint64_t bar_vraw;               // grouped-query decode: a V tile that still needs its tail rows cleared
     // per item parity and row: {max in use (float bits), index of the tile it was decided for};
     // written with one 8-byte store by the tile's owner, polled by the owner of the next tile
-    __shared__ __align__(8) uint2 m_slot[2][128];
+    __shared__ __align__(8) uint2 m_slot[2][ROWS];
     // per item parity, group and row: final reference max and partial row sum of a softmax thread
-    __shared__ float xm[2][2][128], xsum[2][2][128];
+    __shared__ float xm[2][2][ROWS], xsum[2][2][ROWS];
     __shared__ __align__(8) uint64_t bar_stats[2], bar_stats_free[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
@@ -302,7 +307,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         abort_flag = 0;
         fence_mbar_init();
     }
-    if (tid < 256) m_slot[tid >> 7][tid & 127] = make_uint2(0u, 0xFFFFFFFFu);   // no tile has this index
+    if (tid < 2 * ROWS) m_slot[tid / ROWS][tid % ROWS] = make_uint2(0u, 0xFFFFFFFFu);   // no tile has this index
     if constexpr (GQA) {
         // decode: a Q load only writes the rows that carry a (token, head) pair; the other rows of the
         // query tile are zero for the whole launch
@@ -397,7 +402,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const int pages_j = pages;
                 if constexpr (decltype(paged)::value) pages = cache_pages(it, j + 1);
                 // the slot was last read by Q K^T of tile g - NK
-                if (g >= NK && !mbar_wait(smem_u32(&bar_qk[(g - NK) % kRing]), ((g - NK) / kRing) & 1, ctl, kBarKEmpty)) { ok = false; break; }
+                const int ak = SMALL && !V8 ? gq.ahead : NK;
+                if (g >= ak && !mbar_wait(smem_u32(&bar_qk[(g - ak) % kRing]), ((g - ak) / kRing) & 1, ctl, kBarKEmpty)) { ok = false; break; }
                 if constexpr (GQA) {
                     load_cache_tile(k_s + sk * L::kKBytes, L::kKBytes, &tm_k, smem_u32(&bar_kf[sk]), it, j, pages_j, paged);
                 } else {
@@ -448,7 +454,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 } else {
                     const int sv = g % NV;
                     // the slot was last read by P V of tile g - NV
-                    if (g >= NV && !mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
+                    const int av = SMALL ? gq.ahead : NV;
+                    if (g >= av && !mbar_wait(smem_u32(&bar_pvd[(g - av) % kRing]), ((g - av) / kRing) & 1, ctl, kBarVEmpty)) { ok = false; break; }
                     const uint32_t vdst = v_s + sv * L::kVBytes;
                     if constexpr (GQA) {
                         // Rows of the sequence's last tile past its end are stale cache contents when the
@@ -700,10 +707,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // a: the group that had the item's even tiles (SPLIT: so that the result does not depend on where
             // in the CTA's tile sequence the item lies)
             const int ga = SPLIT ? g & 1 : 0;
-            const float m_a = xm[par][ga][r_in_tile], m_b = xm[par][ga ^ 1][r_in_tile];
+            const int r_stat = SMALL ? min(r_in_tile, ROWS - 1) : r_in_tile;   // rows past them are not live
+            const float m_a = xm[par][ga][r_stat], m_b = xm[par][ga ^ 1][r_stat];
             const float m_fin = fmaxf(m_a, m_b);
-            const float l_run = xsum[par][ga][r_in_tile] * ex2_approx(m_a - m_fin) +
-                                xsum[par][ga ^ 1][r_in_tile] * ex2_approx(m_b - m_fin);
+            const float l_run = xsum[par][ga][r_stat] * ex2_approx(m_a - m_fin) +
+                                xsum[par][ga ^ 1][r_stat] * ex2_approx(m_b - m_fin);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_stats_free[par]));
             float inv_l = 1.0f / l_run;
@@ -785,7 +793,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!direct) gq.lse_part[pidx] = lse_val;
                     else if (gq.lse_final != nullptr) gq.lse_final[pidx] = lse_val;
                 }
-                if (!direct || gq.live_rows <= 32) {
+                if (SMALL || !direct || gq.live_rows <= 32) {
 #pragma unroll 1
                     for (int c = 0; c < D / 32; c++) {
                         uint32_t o[32];
@@ -872,8 +880,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int r_in_tile = (warp & 3) * 32 + lane;     // 0..127 == TMEM lane; one thread owns the whole row
         const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t t_o = tmem + lane_off + O_COL + (SPLIT ? grp * D : 0);
-        if (GQA && gq.live_rows <= 16) {
-            // Decode with at most 16 live rows.  As below only the first warp of each group has work, but it
+        if constexpr (SMALL) {
+            // As below only the first warp of each group has work, but it
             // takes its rows through the 16-lane TMEM shapes, which spread a row over four threads: 32 exponentials
             // a thread and tile (64 with more than 8 rows) instead of 128.  Both groups' working warps share one
             // scheduler, and 256 exponentials per pair of tiles on its MUFU were the longest stage of decode over
@@ -1245,8 +1253,8 @@ int launch_instance(const fa_prefill_args& a, DeviceState* st, const CUtensorMap
     GqaDev order{};
     order.group = heads_per_group(n_bh, a.seq_len, a.d_head, FP8 ? 1 : 2);
     const bool grouped = order.group < n_bh;
-    auto kernel = grouped ? prefill_kernel<D, CAUSAL, BF16, FP8, false, true>
-                          : prefill_kernel<D, CAUSAL, BF16, FP8, false, false>;
+    auto kernel = grouped ? prefill_kernel<D, CAUSAL, BF16, FP8, false, true, false>
+                          : prefill_kernel<D, CAUSAL, BF16, FP8, false, false, false>;
     static bool configured[64][2] = {};
     if (!configured[st->device][grouped]) {
         FA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
@@ -1264,11 +1272,11 @@ int launch_instance(const fa_prefill_args& a, DeviceState* st, const CUtensorMap
                             st->status, order);
 }
 
-template <int D, bool BF16, bool FP8>
+template <int D, bool BF16, bool FP8, bool SMALL>
 int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& tq, const CUtensorMap& tk,
                         const CUtensorMap& tv, const CUtensorMap& to) {
-    using L = PrefillSmem<D, FP8>;
-    auto kernel = prefill_kernel<D, false, BF16, FP8, true, false>;
+    using L = PrefillSmem<D, FP8, FP8, SMALL>;
+    auto kernel = prefill_kernel<D, false, BF16, FP8, true, false, SMALL>;
     static bool configured[64] = {};
     if (!configured[st->device]) {
         FA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
@@ -1287,12 +1295,17 @@ int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& 
     // (134 MB of cache, 16 query tiles): 301 us over all heads, 269 us 8 heads at a time.  A single query
     // tile reads everything once, in any order.
     const int walk = n_qt > 1 ? heads_per_group(n_bh, g.kv_len, g.d_head, FP8 ? 1 : 2) : n_bh;
+    // SMALL, 16-bit cache: how many of the stages to use.  All of them where CTAs are left alone with long
+    // sequences while the rest have finished (lengths differ, at most two items a CTA): one CTA then gets
+    // more of the bandwidth (B=16 Hkv=8 Skv<=4096 D=128 paged 37.5 -> 32.9 us, not paged 34.2 -> 32.3).  When
+    // every SM streams to the end the deeper queues cost DRAM efficiency (B=32 Hkv=8 Skv=16384 312 -> 326).
+    const int ahead = g.seq_lens != nullptr && n_items <= 2ll * st->sm_count ? L::NK : L::NK / 3 * 2;
     const int last_heads = n_bh % walk ? n_bh % walk : walk;
     const GqaDev gq{g.o_part, g.lse_part, static_cast<uint16_t*>(g.o_final), g.lse_final, g.n_splits,
                     g.tiles_per_split, g.group, g.n_kv_heads,
                     g.n_tok, tok_per_tile, n_qt, tok_per_tile * g.group, walk,
                     FastDiv(g.n_splits), FastDiv((uint32_t)walk * n_qt), FastDiv(walk), FastDiv(last_heads), FastDiv(g.n_kv_heads), g.seq_lens, g.block_table, g.table_stride,
-                    page_shift};
+                    page_shift, ahead};
     return launch_dependent(kernel, grid, kThreads, L::kTotal, g.stream, 1, tq, tk, tv, to, nullptr, g.kv_len, n_bh, 1,
                             (int)n_items, g.scale * kLog2e, g.q_scale, g.k_scale, g.v_scale, st->status, gq);
 }
@@ -1357,11 +1370,14 @@ int launch_decode_gqa(const GqaLaunch& g, DeviceState* st) {
                                  g.head_stride, bstride, box_cols, box_rows)) != FA_OK) return rc;
     if ((rc = make_tensor_map_4d(&tv, g.v, g.dtype, g.d_head, rows, g.n_kv_heads, blocks, g.row_stride,
                                  g.head_stride, bstride, box_cols, box_rows)) != FA_OK) return rc;
-    if (e4m3) return launch_gqa_instance<128, true, true>(g, st, tq, tk, tv, to);
+    const int tok_per_tile = kBM / g.group < g.n_tok ? kBM / g.group : g.n_tok;
+    const bool small = tok_per_tile * g.group <= 16;
     const bool bf = g.dtype == FA_DTYPE_BF16;
-    if (g.d_head == 64)
-        return bf ? launch_gqa_instance<64, true, false>(g, st, tq, tk, tv, to) : launch_gqa_instance<64, false, false>(g, st, tq, tk, tv, to);
-    return bf ? launch_gqa_instance<128, true, false>(g, st, tq, tk, tv, to) : launch_gqa_instance<128, false, false>(g, st, tq, tk, tv, to);
+#define FA_GQA(DH, BF, F8) (small ? launch_gqa_instance<DH, BF, F8, true>(g, st, tq, tk, tv, to) : launch_gqa_instance<DH, BF, F8, false>(g, st, tq, tk, tv, to))
+    if (e4m3) return FA_GQA(128, true, true);
+    if (g.d_head == 64) return bf ? FA_GQA(64, true, false) : FA_GQA(64, false, false);
+    return bf ? FA_GQA(128, true, false) : FA_GQA(128, false, false);
+#undef FA_GQA
 }
 
 

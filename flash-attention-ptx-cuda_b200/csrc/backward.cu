@@ -548,58 +548,58 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bar_p1[g]));
-                    continue;
-                }
+                } else {
 #pragma unroll
-                for (int c = 0; c < 2; c++) {               // 16 columns of each product at a time
-                    uint32_t sv[16], dv[16];
-                    tmem_ld16x2_wait(tb + c * 16, sv, tb + kW + c * 16, dv);
-                    if (c == 1) {
-                        // the product buffer is free for this parity's next step
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&bar_tfree[g]));
-                    }
-                    if (need_mask) {
+                    for (int c = 0; c < 2; c++) {               // 16 columns of each product at a time
+                        uint32_t sv[16], dv[16];
+                        tmem_ld16x2_wait(tb + c * 16, sv, tb + kW + c * 16, dv);
+                        if (c == 1) {
+                            // the product buffer is free for this parity's next step
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(smem_u32(&bar_tfree[g]));
+                        }
+                        if (need_mask) {
 #pragma unroll
-                        for (int e = 0; e < 16; e++) {
-                            const int cg = c0 + half * 32 + c * 16 + e;     // global index of the streamed row
-                            const bool valid = (MODE == 0) ? (r_glob <= cg) : (cg < seq_len && (!CAUSAL || cg <= r_glob));
-                            sv[e] = valid ? sv[e] : 0xff800000u;    // -inf
+                            for (int e = 0; e < 16; e++) {
+                                const int cg = c0 + half * 32 + c * 16 + e;     // global index of the streamed row
+                                const bool valid = (MODE == 0) ? (r_glob <= cg) : (cg < seq_len && (!CAUSAL || cg <= r_glob));
+                                sv[e] = valid ? sv[e] : 0xff800000u;    // -inf
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < 16; e += 2) {
+                            uint64_t neg_l2 = row_neg_l2, neg_dl = row_neg_dl;
+                            if (MODE == 0) {                    // per column: one 16-byte shared load per pair
+                                const float4 st = *reinterpret_cast<const float4*>(st_neg[MODE == 0 ? warp : 0][i & 1][c * 8 + (e >> 1)]);
+                                neg_l2 = pack2(st.x, st.y);
+                                neg_dl = pack2(st.z, st.w);
+                            }
+                            // p = 2^(s * scale * log2e - lse * log2e);  dS = p * (dP * scale - delta * scale)
+                            const uint64_t x = fma2(pack2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale_log2_2, neg_l2);
+                            float x0, x1;
+                            unpack2(x, x0, x1);
+                            const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
+                            const uint64_t gg = fma2(pack2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), scale2, neg_dl);
+                            float e0, e1;
+                            unpack2(mul2(pack2(p0, p1), gg), e0, e1);
+                            pk[c * 8 + (e >> 1)] = pack_16<BF16>(p0, p1);
+                            dk[c * 8 + (e >> 1)] = pack_16<BF16>(e0, e1);
                         }
                     }
-#pragma unroll
-                    for (int e = 0; e < 16; e += 2) {
-                        uint64_t neg_l2 = row_neg_l2, neg_dl = row_neg_dl;
-                        if (MODE == 0) {                    // per column: one 16-byte shared load per pair
-                            const float4 st = *reinterpret_cast<const float4*>(st_neg[MODE == 0 ? warp : 0][i & 1][c * 8 + (e >> 1)]);
-                            neg_l2 = pack2(st.x, st.y);
-                            neg_dl = pack2(st.z, st.w);
-                        }
-                        // p = 2^(s * scale * log2e - lse * log2e);  dS = p * (dP * scale - delta * scale)
-                        const uint64_t x = fma2(pack2(__uint_as_float(sv[e]), __uint_as_float(sv[e + 1])), scale_log2_2, neg_l2);
-                        float x0, x1;
-                        unpack2(x, x0, x1);
-                        const float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-                        const uint64_t gg = fma2(pack2(__uint_as_float(dv[e]), __uint_as_float(dv[e + 1])), scale2, neg_dl);
-                        float e0, e1;
-                        unpack2(mul2(pack2(p0, p1), gg), e0, e1);
-                        pk[c * 8 + (e >> 1)] = pack_16<BF16>(p0, p1);
-                        dk[c * 8 + (e >> 1)] = pack_16<BF16>(e0, e1);
+                    // the operand columns of this parity were read by the accumulations of step T-2
+                    if (T >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc))) {
+                        ok = false;
+                        break;
                     }
+                    const uint32_t op_off = half * 16u;         // each half writes its 16 columns of pairs
+                    if (MODE == 0) tmem_st_x16(tmem + lane_off + OPP0 + g * OP_STRIDE + op_off, pk);
+                    tmem_st_x16(tmem + lane_off + OPD0 + g * OP_STRIDE + op_off, dk);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&bar_p[g]));
                 }
-                // the operand columns of this parity were read by the accumulations of step T-2
-                if (T >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc))) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t op_off = half * 16u;         // each half writes its 16 columns of pairs
-                if (MODE == 0) tmem_st_x16(tmem + lane_off + OPP0 + g * OP_STRIDE + op_off, pk);
-                tmem_st_x16(tmem + lane_off + OPD0 + g * OP_STRIDE + op_off, dk);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bar_p[g]));
             }
             if (!ok) break;
             BwdItem nx;

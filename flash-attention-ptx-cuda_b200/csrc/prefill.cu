@@ -16,18 +16,17 @@
 //
 // d_head 64 (prefill) splits O and the P V issue by softmax group, as described at SPLIT below;
 // the rest of this list is the general form.
-//   warps 8, 11        TMA producers (one lane each): Q per item and the K tiles / the V
-//   (one lane each)    tiles (128 keys) through mbarrier-guarded shared-memory rings,
-//                      128-byte swizzle.  K and V have a producer each so that K loads
-//                      are not held back behind the later-freed V slots.
-//   warp 9             issues S = Q K^T (tcgen05.mma, lane 0) into one of THREE score
-//                      buffers in TMEM, used round-robin; it waits for the tile's K and
-//                      for the P V that last read the buffer (three tiles back).
+//   warps 8, 11        TMA producers: Q per item and the K tiles / the V tiles (128 keys)
+//                      through mbarrier-guarded shared-memory rings, 128-byte swizzle.
+//                      K and V have a producer each so that K loads are not held back
+//                      behind the later-freed V slots.
+//   warp 9             issues S = Q K^T (tcgen05.mma) into one of THREE score buffers in
+//                      TMEM, used round-robin; it waits for the tile's K and for the P V
+//                      that last read the buffer (three tiles back).
 //   warp 10            issues O += P V: P from TMEM, V (MN-major) from shared memory.
-//                      Q K^T and P V have an issuer each because every tcgen05.mma /
-//                      commit costs its issuing thread ~50-100 clocks; one thread doing
-//                      both was the bottleneck.  Each issuer commits once per tile, onto a
-//                      ring of completion barriers that every interested party waits on
+//                      Producers and issuers walk their loops as whole warps and one
+//                      elected lane issues (elect_one, ptx.cuh).  Each issuer commits once
+//                      per tile, onto a ring of completion barriers that every interested party waits on
 //                      (softmax: S is there; K producer: slot free / Q K^T issuer: score
 //                      buffer free; V producer: slot free; softmax: O may be rescaled).
 //   warps 0-7          softmax, two groups of four warps.  Group 0 owns the even key
@@ -399,7 +398,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if constexpr (decltype(paged)::value) pages = cache_pages(it, 0);
             for (int j = 0; j < it.n_kv; j++, g++) {
                 const int sk = g % NK;
-                const int pages_j = pages;
+                [[maybe_unused]] const int pages_j = pages;
                 if constexpr (decltype(paged)::value) pages = cache_pages(it, j + 1);
                 // the slot was last read by Q K^T of tile g - NK
                 const int ak = SMALL && !V8 ? gq.ahead : NK;
@@ -436,7 +435,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     } else if (!SPLIT && warp == 11) {
         // ------------------------------------------------------------ TMA producer: V
         auto produce = [&](auto paged) {
-        int g = 0, n_scrub = 0;
+        int g = 0;
+        [[maybe_unused]] int n_scrub = 0;
         bool ok = true;
         for (int r = 0; ok && r < n_rounds; r++) {
             Item it;
@@ -444,7 +444,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             int pages = -1;
             if constexpr (decltype(paged)::value) pages = cache_pages(it, 0);
             for (int j = 0; j < it.n_kv; j++, g++) {
-                const int pages_j = pages;
+                [[maybe_unused]] const int pages_j = pages;
                 if constexpr (decltype(paged)::value) pages = cache_pages(it, j + 1);
                 if constexpr (V8) {
                     // e4m3 V lands in its own buffers; warps 12-15 turn it into the fp16 operand.

@@ -315,17 +315,17 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
             bool issued = false;
             for (int t = (g ^ gs) & 1; t < it.n_steps; t += 2) {
                 const int T = gs + t, s = T % kStages;
+                LaneWaits lw;
                 // the tiles arrived long ago; the buffer is what the issue waits for
-                if (!mbar_wait(smem_u32(&bar_full[s]), (T / kStages) & 1, ctl, kBwdBarFull)) { ok = false; break; }
+                mbar_wait(lw, smem_u32(&bar_full[s]), (T / kStages) & 1, ctl, kBwdBarFull);
                 if (T >= 2) {
                     // products of step T reuse the TMEM buffer of step T-2
-                    if (INPLACE) ok = mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
-                    else         ok = mbar_wait(smem_u32(&bar_tfree[g]), ((T >> 1) - 1) & 1, ctl, kBwdBarFree);
-                    if (!ok) break;
+                    if (INPLACE) mbar_wait(lw, smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
+                    else         mbar_wait(lw, smem_u32(&bar_tfree[g]), ((T >> 1) - 1) & 1, ctl, kBwdBarFree);
                 }
                 tc_fence_after();
                 const uint64_t db0 = make_sdesc(b_s + s * 2 * L::kTileB, hi_k), db1 = db0 + (L::kTileB >> 4);
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
@@ -336,10 +336,10 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 if (INPLACE) {
                     __syncwarp();
                     // the dP^T half has a chain of its own: dK of step T - 2, not dV, must be done
-                    if (T >= 2 && !mbar_wait(smem_u32(&bar_acc1[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc)) { ok = false; break; }
+                    if (T >= 2) mbar_wait(lw, smem_u32(&bar_acc1[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
                     tc_fence_after();
                 }
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
@@ -347,7 +347,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     }
                     tc_commit(smem_u32(INPLACE ? &bar_t1[g] : &bar_t[g]));
                 }
-                __syncwarp();
+                if (!warp_all(lw.ok)) { ok = false; break; }
                 issued = true;
             }
             if (!ok) break;
@@ -375,20 +375,21 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
         for (int k = 0; ok && bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
             for (int t = 0; t < it.n_steps; t++) {
                 const int T = gs + t, s = T % kStages, g = T & 1;
-                if (!mbar_wait(smem_u32(INPLACE && x == 1 ? &bar_p1[g] : &bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP)) { ok = false; break; }
+                LaneWaits lw;
+                mbar_wait(lw, smem_u32(INPLACE && x == 1 ? &bar_p1[g] : &bar_p[g]), (T >> 1) & 1, ctl, kBwdBarP);
                 // the accumulators of the item before must have been read out
-                if (t == 0 && k >= 1 && !mbar_wait(smem_u32(&bar_accfree), (k - 1) & 1, ctl, kBwdBarFree)) { ok = false; break; }
+                if (t == 0 && k >= 1) mbar_wait(lw, smem_u32(&bar_accfree), (k - 1) & 1, ctl, kBwdBarFree);
                 tc_fence_after();
                 const uint64_t db = make_sdesc(b_s + s * 2 * L::kTileB + (use_p ? L::kTileB : 0), hi_mn);
                 const uint32_t op = op0 + g * OP_STRIDE;
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
 #pragma unroll
                     for (int kk = 0; kk < kW / 16; kk++)
                         mma_f16_ts(acc, op + op16_col(kk, INPLACE), db + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
                     tc_commit(smem_u32(INPLACE && x == 1 ? &bar_acc1[s] : &bar_acc[s]));
                     if (t == it.n_steps - 1) tc_commit(smem_u32(&bar_done));
                 }
-                __syncwarp();
+                if (!warp_all(lw.ok)) { ok = false; break; }
             }
             gs += it.n_steps;
         }
@@ -397,7 +398,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
         BwdItem it;
         for (int k = 0; bwd_item<CAUSAL, MODE>(k, n_items, n_bh, n_tiles, seq_len, it); k++) {
             const int buf = k % NA;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_ostaged), k & 1, ctl, kBwdBarDone))) break;
+            if (!mbar_wait(smem_u32(&bar_ostaged), k & 1, ctl, kBwdBarDone)) break;
             if (lane == 0) {
                 const uint32_t o_s = base + buf * 2 * L::kTile;
                 for (int b = 0; b < NBOX; b++) {
@@ -482,7 +483,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 const int T = gs + t, i = T >> 1;
                 const int c0 = row0 + t * kW;               // first streamed row (= column of T0/T1) of the step
                 const uint32_t tb = tmem + lane_off + g * 128 + half * 32;
-                ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_t[g]), i & 1, ctl, kBwdBarT));
+                ok = ok && mbar_wait(smem_u32(&bar_t[g]), i & 1, ctl, kBwdBarT);
                 if (!ok) break;
                 if (MODE == 0) {
                     stage_stats((i + 1) & 1, nx_l2, nx_dl);
@@ -527,7 +528,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&bar_p[g]));
-                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_t1[g]), i & 1, ctl, kBwdBarT));
+                    ok = mbar_wait(smem_u32(&bar_t1[g]), i & 1, ctl, kBwdBarT);
                     if (!ok) break;
                     tc_fence_after();
                     uint32_t dv[32];
@@ -588,7 +589,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                         }
                     }
                     // the operand columns of this parity were read by the accumulations of step T-2
-                    if (T >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc))) {
+                    if (T >= 2 && !mbar_wait(smem_u32(&bar_acc[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc)) {
                         ok = false;
                         break;
                     }
@@ -609,7 +610,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 if (MODE == 0) prefetch(nx, gs + n_steps, 1, pf2_l2, pf2_dl);
             }
             // ---- accumulators -> 16-bit -> global, 32 columns per group of four warps at a time
-            ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_done), k & 1, ctl, kBwdBarDone));
+            ok = ok && mbar_wait(smem_u32(&bar_done), k & 1, ctl, kBwdBarDone);
             if (ok) {
                 tc_fence_after();
 #pragma unroll 1

@@ -50,6 +50,28 @@ FA_HOST_DEVICE int bounded_wait(Poll poll, Aborted aborted, Clock now_ns, unsign
     return kWaitDone;
 }
 
+// Waits made by all lanes of a warp.  The lanes' answers can differ: one sees the phase complete while another
+// runs out of time or sees the abort flag.  A warp that left its loop lane by lane on them would split, and
+// those that stay would wait without limit, at the next full-mask instruction, for those that left.  So the
+// warp votes; `all(x)` is true in every lane if x is true in all of them.
+//
+// The plain form votes on each wait: every lane gets the same answer.
+template <class Wait, class All>
+FA_HOST_DEVICE bool warp_wait(Wait wait, All all) {
+    return all(wait());
+}
+// Where one elected lane issues MMAs, the vote comes after the issue, off its path: the lanes note what their
+// waits said, the elected lane issues if all of its own succeeded (what it issues is ready then), and
+// `all(ok)` decides for all of them whether the loop goes on.  A vote on each wait before the issue cost
+// another 0.5 % at d_head 128 (bf16 B*H=32 S=8192 no mask: 975 us, 970 this way, 963 without any vote).
+struct LaneWaits {
+    bool ok = true;
+    template <class Wait>
+    FA_HOST_DEVICE void wait(Wait w) {
+        if (!w()) ok = false;
+    }
+};
+
 // The status word a waiter records when it gives up on barrier `barrier_id`.
 FA_HOST_DEVICE int wait_timeout_word(int barrier_id) { return (kErrWaitTimeout << 16) | (barrier_id & 0xFFFF); }
 

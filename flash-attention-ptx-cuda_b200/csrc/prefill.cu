@@ -514,14 +514,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (!mbar_wait(smem_u32(&bar_qf), it_n & 1, ctl, kBarQFull)) break;
             for (int j = 0; j < it.n_kv; j++, g++) {
                 const int sk = g % NK;
-                if (!mbar_wait(smem_u32(&bar_kf[sk]), (g / NK) & 1, ctl, kBarKFull)) { ok = false; break; }
+                LaneWaits lw;
+                mbar_wait(lw, smem_u32(&bar_kf[sk]), (g / NK) & 1, ctl, kBarKFull);
                 // the score buffer last held S and then P of tile g - kNU: that P V must be done
-                if (g >= kNU && !mbar_wait(smem_u32(&bar_pvd[(g - kNU) % kRing]), ((g - kNU) / kRing) & 1, ctl, kBarSFree)) { ok = false; break; }
+                if (g >= kNU) mbar_wait(lw, smem_u32(&bar_pvd[(g - kNU) % kRing]), ((g - kNU) / kRing) & 1, ctl, kBarSFree);
                 tc_fence_after();
                 const uint32_t kb = k_s + sk * L::kKBytes;
                 const uint32_t sc = tmem + u * 128;
                 const uint64_t dk = make_sdesc(kb, hi_k);
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
                     if constexpr (FP8) {
 #pragma unroll
                         for (int kk = 0; kk < D / 32; kk++)          // 32 e4m3 (32 bytes) of d_head per MMA
@@ -536,7 +537,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     tc_commit(smem_u32(&bar_qk[g % kRing]));                // S is ready; the K slot is free
                     if (j == it.n_kv - 1) tc_commit(smem_u32(&bar_qe));   // Q is dead after the item's last Q K^T
                 }
-                __syncwarp();
+                if (!warp_all(lw.ok)) { ok = false; break; }
                 u = (u == kNU - 1) ? 0 : u + 1;
             }
             it_n++;
@@ -559,22 +560,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             for (int j = j0; j < it.n_kv; j += 2) {
                 const int g = g0 + j;
                 const int sv = g % NV;
-                if (!mbar_wait(smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull)) { ok = false; break; }
-                if (!mbar_wait(smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull)) { ok = false; break; }
+                LaneWaits lw;
+                mbar_wait(lw, smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull);
+                mbar_wait(lw, smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull);
                 // the first P V of an item overwrites O: the epilogue of the last item must have read it
-                if (j == j0 && used > 0 && !mbar_wait(smem_u32(&bar_ofree[par]), (used - 1) & 1, ctl, kBarOFree)) { ok = false; break; }
+                if (j == j0 && used > 0) mbar_wait(lw, smem_u32(&bar_ofree[par]), (used - 1) & 1, ctl, kBarOFree);
                 tc_fence_after();
                 const uint32_t vb = v_s + sv * L::kVBytes;
                 const uint32_t pc = tmem + u * 128;         // P overwrote the first 64 columns of the tile's S
                 const uint64_t dv = make_sdesc(vb, hi_v);
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
 #pragma unroll
                     for (int kk = 0; kk < kBN / 16; kk++)
                         mma_f16_ts(oc, pc + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > j0 || kk > 0) ? 1u : 0u);
                     tc_commit(smem_u32(&bar_pvd[g % kRing]));               // score buffer and V slot are free
                     if (j + 2 >= it.n_kv) tc_commit(smem_u32(&bar_odone[par]));   // the item's accumulator is complete
                 }
-                __syncwarp();
+                if (!warp_all(lw.ok)) { ok = false; break; }
                 u += 2;
                 if (u >= kNU) { u -= kNU; u_phase ^= 1; }
             }
@@ -592,22 +594,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (!get_item<CAUSAL, GQA, GROUPED>(r, n_items, n_bh, n_qtiles, seq_len, gq, it)) continue;
             for (int j = 0; j < it.n_kv; j++, g++) {
                 const int sv = g % NV;
-                if (!mbar_wait(smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull)) { ok = false; break; }
-                if (!mbar_wait(smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull)) { ok = false; break; }
+                LaneWaits lw;
+                mbar_wait(lw, smem_u32(&bar_vf[sv]), (g / NV) & 1, ctl, kBarVFull);
+                mbar_wait(lw, smem_u32(&bar_pf[u]), u_phase, ctl, kBarPFull);
                 // the first P V of an item overwrites O: the previous item's epilogue must have read it
-                if (j == 0 && it_n > 0 && !mbar_wait(smem_u32(&bar_ofree[0]), (it_n - 1) & 1, ctl, kBarOFree)) { ok = false; break; }
+                if (j == 0 && it_n > 0) mbar_wait(lw, smem_u32(&bar_ofree[0]), (it_n - 1) & 1, ctl, kBarOFree);
                 tc_fence_after();
                 const uint32_t vb = v_s + sv * L::kVBytes;
                 const uint32_t pc = tmem + u * 128;         // P overwrote the first 64 columns of the tile's S
                 const uint64_t dv = make_sdesc(vb, hi_v);
-                if (elect_one()) {
+                if (elect_one() && lw.ok) {
 #pragma unroll
                     for (int kk = 0; kk < kBN / 16; kk++)
                         mma_f16_ts(tmem + O_COL, pc + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
                     tc_commit(smem_u32(&bar_pvd[g % kRing]));               // score buffer and V slot are free
                     if (j == it.n_kv - 1) tc_commit(smem_u32(&bar_odone[0]));   // the item's O is complete
                 }
-                __syncwarp();
+                if (!warp_all(lw.ok)) { ok = false; break; }
                 if (u == kNU - 1) { u = 0; u_phase ^= 1; } else { u++; }
             }
             it_n++;
@@ -624,7 +627,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         auto rendezvous4 = [&](uint32_t parity) -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_epi));
-            return __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_epi), parity, ctl, kBarEpi));
+            return mbar_wait(smem_u32(&bar_epi), parity, ctl, kBarEpi);
         };
         int it_n = 0, g = 0;
         uint32_t used = 0;                                // SPLIT: bit x: parity of the items accumulator x has had (g: first tile of the item)
@@ -656,7 +659,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     bool w = mbar_wait(smem_u32(&bar_v8f[s8]), (g / L::NV8) & 1, ctl, kBarV8Full);
                     // the fp16 buffer must have been consumed by the P V that last read it
                     if (g >= NV) w = w && mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty);
-                    if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
+                    if (!w) { ok = false; break; }
                     const uint32_t src_base = v8_s + s8 * L::kV8Bytes;
                     const uint32_t dst_base = v_s + sv * L::kVBytes;
                     // decode over a cache: rows past the sequence's end may hold stale bytes (NaN codes
@@ -703,7 +706,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             // ---- epilogue of the item
             const int par = it_n & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats[par]), (it_n >> 1) & 1, ctl, kBarStats))) break;
+            if (!mbar_wait(smem_u32(&bar_stats[par]), (it_n >> 1) & 1, ctl, kBarStats)) break;
             // a: the group that had the item's even tiles (SPLIT: so that the result does not depend on where
             // in the CTA's tile sequence the item lies)
             const int ga = SPLIT ? g & 1 : 0;
@@ -726,7 +729,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 bool w = mbar_wait(smem_u32(&bar_odone[ga]), (used >> ga) & 1, ctl, kBarODone);
                 if (has_b) w = w && mbar_wait(smem_u32(&bar_odone[ga ^ 1]), (used >> (ga ^ 1)) & 1, ctl, kBarODone);
                 used ^= has_b ? 3u : 1u << ga;
-                if (!__all_sync(0xffffffffu, w)) break;
+                if (!w) break;
                 tc_fence_after();
                 // the staging buffer must have been drained by the previous item's TMA store
                 if (tid == 384) tma_store_wait_read();
@@ -772,7 +775,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 it_n++;
                 continue;
             }
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_odone[0]), it_n & 1, ctl, kBarODone))) break;
+            if (!mbar_wait(smem_u32(&bar_odone[0]), it_n & 1, ctl, kBarODone)) break;
             tc_fence_after();
             bool seen = true;
             if constexpr (GQA) {
@@ -904,7 +907,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 for (int j = (g0 & 1) == grp ? 0 : 1; j < it.n_kv; j += 2) {
                     const int g = g0 + j, u = g % kNU;
                     const int kv_start = (it.t0 + j) * kBN;
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, kBarSFull))) { ok = false; break; }
+                    if (!mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, kBarSFull)) { ok = false; break; }
                     tc_fence_after();
                     if (idle) {
                         tc_fence_before();
@@ -975,7 +978,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     m0 = n0;
                     m1 = n1;
                     if (__any_sync(0xffffffffu, changed)) {       // rare: rescale O before this tile's P V
-                        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, kBarPV))) { ok = false; break; }
+                        if (!mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, kBarPV)) { ok = false; break; }
                         tc_fence_after();
                         const float r0 = __shfl_sync(0xffffffffu, f0, (lane & 7) * 4), r1 = __shfl_sync(0xffffffffu, f1, (lane & 7) * 4);
                         const float factor = lane < 8 ? r0 : lane < 16 ? r1 : 1.0f;   // of TMEM lane `lane`
@@ -1020,7 +1023,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (!ok) break;
                 const int par = it_n & 1;
                 if (it_n >= 2 &&
-                    !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, kBarStatsFree))) { ok = false; break; }
+                    !mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, kBarStatsFree)) { ok = false; break; }
                 if (!idle) {
                     float a, b, c, d;
                     unpack2(sum0, a, b);
@@ -1072,8 +1075,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             for (int j = (g0 & 1) == grp ? 0 : 1; j < it.n_kv; j += 2) {
                 const int g = g0 + j;                     // global tile index; g & 1 == grp
                 const int kv_start = (GQA ? it.t0 + j : j) * kBN;
-                // The votes keep the warp together: every lane leaves the loop or none does.
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, kBarSFull))) { ok = false; break; }
+                // Every lane leaves the loop or none does (warp_wait, bounded_wait.h).
+                if (!mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, kBarSFull)) { ok = false; break; }
                 tc_fence_after();
                 const int u = g % kNU;                    // the tile's score buffer; P goes back into its first half
                 const uint32_t t_s = tmem + lane_off + u * 128;
@@ -1153,7 +1156,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // ---- rare: the max in use grew -> rescale O in TMEM before this tile's P V
                 if (__any_sync(0xffffffffu, changed)) {
                     // the P V before this one must have finished accumulating into O
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - NO) % kRing]), ((g - NO) / kRing) & 1, ctl, kBarPV))) { ok = false; break; }
+                    if (!mbar_wait(smem_u32(&bar_pvd[(g - NO) % kRing]), ((g - NO) / kRing) & 1, ctl, kBarPV)) { ok = false; break; }
                     tc_fence_after();
                     // rows whose max did not change multiply by one; m_mine is not the previous max of
                     // the ROW (the other thread may have moved it), so the factor comes from m_prev
@@ -1212,7 +1215,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // go straight on to the next item
                 const int par = it_n & 1;
                 if (it_n >= 2 &&
-                    !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, kBarStatsFree))) { ok = false; break; }
+                    !mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, kBarStatsFree)) { ok = false; break; }
                 float l0, l1;
                 unpack2(lsum2, l0, l1);
                 xm[par][grp][r_in_tile] = m_mine;

@@ -226,16 +226,19 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int r = 0; ok && r < n_rounds; r++) {
                 Item2 it;
                 if (!get_item2<CAUSAL>(r, n_items, n_bh, n_pairs, seq_len, heads_per_group, it)) continue;
-                if (!mbar_wait_cluster(smem_u32(&bar_qf), it_n & 1, ctl, k2QFull)) break;
+                LaneWaits lq;
+                mbar_wait_cluster(lq, smem_u32(&bar_qf), it_n & 1, ctl, k2QFull);
+                if (!warp_all(lq.ok)) break;
                 for (int j = 0; j < it.n_kv; j++, g++) {
                     const int sk = g % kStages;
-                    if (!mbar_wait_cluster(smem_u32(&bar_kf[sk]), (g / kStages) & 1, ctl, k2KFull)) { ok = false; break; }
+                    LaneWaits lw;
+                    mbar_wait_cluster(lw, smem_u32(&bar_kf[sk]), (g / kStages) & 1, ctl, k2KFull);
                     // the score buffer last held S and then P of tile g - kNU: that P V must be done
-                    if (g >= kNU && !mbar_wait(smem_u32(&bar_pvd[(g - kNU) % kRing]), ((g - kNU) / kRing) & 1, ctl, k2SFree)) { ok = false; break; }
+                    if (g >= kNU) mbar_wait(lw, smem_u32(&bar_pvd[(g - kNU) % kRing]), ((g - kNU) / kRing) & 1, ctl, k2SFree);
                     tc_fence_after();
                     const uint64_t dk = make_sdesc(k_s + sk * L::kKHalf, hi_k);
                     const uint32_t sc = tmem + u * 128;
-                    if (elect_one()) {
+                    if (elect_one() && lw.ok) {
 #pragma unroll
                         for (int kk = 0; kk < D / 16; kk++) {
                             const uint32_t qoff = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4;
@@ -244,7 +247,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         }
                         tc_commit_2sm(smem_u32(&bar_qk[g % kRing]));  // both CTAs: S ready, K slot free, (last tile) Q free
                     }
-                    __syncwarp();
+                    if (!warp_all(lw.ok)) { ok = false; break; }
                     u = (u == kNU - 1) ? 0 : u + 1;
                 }
                 it_n++;
@@ -263,20 +266,21 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (!get_item2<CAUSAL>(r, n_items, n_bh, n_pairs, seq_len, heads_per_group, it)) continue;
                 for (int j = 0; j < it.n_kv; j++, g++) {
                     const int sv = g % kStages;
-                    if (!mbar_wait_cluster(smem_u32(&bar_vf[sv]), (g / kStages) & 1, ctl, k2VFull)) { ok = false; break; }
-                    if (!mbar_wait_cluster(smem_u32(&bar_pf[u]), u_phase, ctl, k2PFull)) { ok = false; break; }
+                    LaneWaits lw;
+                    mbar_wait_cluster(lw, smem_u32(&bar_vf[sv]), (g / kStages) & 1, ctl, k2VFull);
+                    mbar_wait_cluster(lw, smem_u32(&bar_pf[u]), u_phase, ctl, k2PFull);
                     // the first P V of an item overwrites O: both CTAs' epilogues must have read the previous one
-                    if (j == 0 && it_n > 0 && !mbar_wait_cluster(smem_u32(&bar_ofree), (it_n - 1) & 1, ctl, k2OFree)) { ok = false; break; }
+                    if (j == 0 && it_n > 0) mbar_wait_cluster(lw, smem_u32(&bar_ofree), (it_n - 1) & 1, ctl, k2OFree);
                     tc_fence_after();
                     const uint64_t dv = make_sdesc(v_s + sv * L::kVHalf, hi_v);
                     const uint32_t pc = tmem + u * 128;
-                    if (elect_one()) {
+                    if (elect_one() && lw.ok) {
 #pragma unroll
                         for (int kk = 0; kk < kBN / 16; kk++)
                             mma_f16_ts_2sm(tmem + O_COL, pc + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
                         tc_commit_2sm(smem_u32(&bar_pvd[g % kRing])); // both CTAs: score buffer and V slot free, (last tile) O done
                     }
-                    __syncwarp();
+                    if (!warp_all(lw.ok)) { ok = false; break; }
                     if (u == kNU - 1) { u = 0; u_phase ^= 1; } else { u++; }
                 }
                 it_n++;
@@ -291,7 +295,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         auto rendezvous4 = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bar_epi));
-            const bool w = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_epi), n_rv & 1, ctl, k2Epi));
+            const bool w = mbar_wait(smem_u32(&bar_epi), n_rv & 1, ctl, k2Epi);
             n_rv++;
             return w;
         };
@@ -302,7 +306,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             g += it.n_kv;
             const int q_start = (2 * it.pair + static_cast<int>(rank)) * kBM;
             const int par = it_n & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats[par]), (it_n >> 1) & 1, ctl, k2Stats))) break;
+            if (!mbar_wait(smem_u32(&bar_stats[par]), (it_n >> 1) & 1, ctl, k2Stats)) break;
             const float m_a = xm[par][0][r_in_tile], m_b = xm[par][1][r_in_tile];
             const float m_fin = fmaxf(m_a, m_b);
             const float l_run = xsum[par][0][r_in_tile] * ex2_approx(m_a - m_fin) +
@@ -314,7 +318,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (lse_out != nullptr && row < seq_len)
                 lse_out[static_cast<size_t>(it.bh) * seq_len + row] = kLn2 * (m_fin + log2f(l_run));
             // O is complete when the item's last P V is
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, k2ODone))) break;
+            if (!mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, k2ODone)) break;
             tc_fence_after();
             if (tid == 384) tma_store_wait_read();        // staging drained by the previous item's store
             if (!rendezvous4()) break;
@@ -376,7 +380,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int j = (g0 & 1) == grp ? 0 : 1; j < it.n_kv; j += 2) {
                 const int g = g0 + j;
                 const int kv_start = j * kBN;
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, k2SFull))) { ok = false; break; }
+                if (!mbar_wait(smem_u32(&bar_qk[g % kRing]), (g / kRing) & 1, ctl, k2SFull)) { ok = false; break; }
                 tc_fence_after();
                 const int u = g % kNU;
                 const uint32_t t_s = tmem + lane_off + u * 128;
@@ -428,7 +432,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 }
                 if (__any_sync(0xffffffffu, changed)) {
                     // P V(g-1) must have finished accumulating into O
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, k2PV))) { ok = false; break; }
+                    if (!mbar_wait(smem_u32(&bar_pvd[(g - 1) % kRing]), ((g - 1) / kRing) & 1, ctl, k2PV)) { ok = false; break; }
                     tc_fence_after();
                     const float factor = changed ? ex2_approx(m_prev_keep - m_new) : 1.0f;
 #pragma unroll 1
@@ -476,7 +480,7 @@ prefill_2sm_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             {
                 const int par = it_n & 1;
                 if (it_n >= 2 &&
-                    !__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, k2StatsFree))) { ok = false; break; }
+                    !mbar_wait(smem_u32(&bar_stats_free[par]), ((it_n >> 1) - 1) & 1, ctl, k2StatsFree)) { ok = false; break; }
                 float l0, l1;
                 unpack2(lsum2, l0, l1);
                 xm[par][grp][r_in_tile] = m_mine;

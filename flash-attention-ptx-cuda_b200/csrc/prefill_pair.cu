@@ -336,17 +336,18 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         // S = Q K^T of query tile X against the item's key tile j (tile t[X] + j of that chain).
         auto issue_qk = [&](int X, int j) -> bool {
             const int gk = g0 + j, sk = gk % NK;
-            if (!mbar_wait(smem_u32(&cb.k_full[sk]), (gk / NK) & 1, ctl, kPKFull)) return false;
+            LaneWaits lw;
+            mbar_wait(lw, smem_u32(&cb.k_full[sk]), (gk / NK) & 1, ctl, kPKFull);
             FA_PROBE(0);
             if constexpr (!INPLACE) {
                 // the softmax must have read the previous scores out of the buffer
-                if (t[X] + j > 0 && !mbar_wait(smem_u32(&cb.s_free[X]), (t[X] + j - 1) & 1, ctl, kPSFree)) return false;
+                if (t[X] + j > 0) mbar_wait(lw, smem_u32(&cb.s_free[X]), (t[X] + j - 1) & 1, ctl, kPSFree);
             }
             tc_fence_after();
             FA_PROBE(1);
             const uint64_t dk = make_sdesc(k_s + sk * L::kTile, hi_k), dq = make_sdesc(q_s + X * L::kTile, hi_k);
             const uint32_t s_t = tmem + (X ? S_COL1 : S_COL0);
-            if (elect_one()) {
+            if (elect_one() && lw.ok) {
 #pragma unroll
                 for (int kk = 0; kk < D / 16; kk++) {
                     const uint32_t off = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4;
@@ -354,32 +355,31 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 }
                 tc_commit(smem_u32(&cb.s_full[X][(t[X] + j) % kRing]));
             }
-            __syncwarp();
             FA_PROBE(2);
-            return true;
+            return warp_all(lw.ok);
         };
         // O += P V of query tile X for the item's key tile j.
         auto issue_pv = [&](int X, int j) -> bool {
             const int gv = g0 + j, sv = gv % NV;
-            if (!mbar_wait(smem_u32(&cb.v_full[sv]), (gv / NV) & 1, ctl, kPVFull)) return false;
+            LaneWaits lw;
+            mbar_wait(lw, smem_u32(&cb.v_full[sv]), (gv / NV) & 1, ctl, kPVFull);
             FA_PROBE(3);
-            if (!mbar_wait(smem_u32(&cb.p_full[X]), (t[X] + j) & 1, ctl, kPPFull)) return false;
+            mbar_wait(lw, smem_u32(&cb.p_full[X]), (t[X] + j) & 1, ctl, kPPFull);
             FA_PROBE(4);
             // the first P V of an item overwrites O: the previous item's epilogue must have read it
-            if (j == 0 && itx[X] > 0 && !mbar_wait(smem_u32(&cb.o_free[X]), (itx[X] - 1) & 1, ctl, kPOFree)) return false;
+            if (j == 0 && itx[X] > 0) mbar_wait(lw, smem_u32(&cb.o_free[X]), (itx[X] - 1) & 1, ctl, kPOFree);
             tc_fence_after();
             FA_PROBE(5);
             const uint64_t dv = make_sdesc(v_s + sv * L::kTile, hi_v);
             const uint32_t p_t = tmem + (X ? P_COL1 : P_COL0), o_t = tmem + (X ? O_COL1 : O_COL0);
-            if (elect_one()) {
+            if (elect_one() && lw.ok) {
 #pragma unroll
                 for (int kk = 0; kk < kBN / 16; kk++)
                     mma_f16_ts(o_t, p_t + kk * 8, dv + kk * (2048 >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
                 tc_commit(smem_u32(&cb.pv_done[X][(t[X] + j) % kRing]));
             }
-            __syncwarp();
             FA_PROBE(6);
-            return true;
+            return warp_all(lw.ok);
         };
 
         bool ok = true;
@@ -418,7 +418,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         auto rendezvous4 = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&cb.epi));
-            const bool w = __all_sync(0xffffffffu, mbar_wait(smem_u32(&cb.epi), n_rv & 1, ctl, kPEpi));
+            const bool w = mbar_wait(smem_u32(&cb.epi), n_rv & 1, ctl, kPEpi);
             n_rv++;
             return w;
         };
@@ -434,12 +434,12 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 if (n_x == 0) continue;
                 tx[X] += n_x;
                 const uint32_t t_o = tmem + lane_off + (X ? O_COL1 : O_COL0);
-                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&cb.stats_full[X]), itx[X] & 1, ctl, kPStatsFull))) { ok = false; break; }
+                if (!mbar_wait(smem_u32(&cb.stats_full[X]), itx[X] & 1, ctl, kPStatsFull)) { ok = false; break; }
                 const float inv_l = cb.inv_l[X][r_in_tile];
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&cb.stats_free[X]));
                 // O is complete when the item's last P V is
-                if (!__all_sync(0xffffffffu, wait_pv_done(X, tx[X] - 1, kPODone))) { ok = false; break; }
+                if (!wait_pv_done(X, tx[X] - 1, kPODone)) { ok = false; break; }
                 tc_fence_after();
                 // the staging tile must have been drained by the bulk store that last read it
                 const int buf = (NO == 2) ? X : 0;
@@ -512,8 +512,8 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             uint64_t lsum2 = pack2(0.0f, 0.0f);
 
             for (int j = 0; j < n_x; j++, t++) {
-                // The votes keep the warp together: every lane leaves the loop or none does.
-                if (!__all_sync(0xffffffffu, wait_qk_done(X, t, kPSFull))) { ok = false; break; }
+                // Every lane leaves the loop or none does (warp_wait, bounded_wait.h).
+                if (!wait_qk_done(X, t, kPSFull)) { ok = false; break; }
                 tc_fence_after();
                 FA_PROBE(0);
                 uint32_t s[128];
@@ -548,7 +548,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                 // ---- rare: the max in use grew -> rescale O in TMEM before this tile's P V
                 if (__any_sync(0xffffffffu, changed)) {
                     if (!pv_waited) {
-                        if (!__all_sync(0xffffffffu, wait_pv_done(X, t - 1, kPPvDone))) { ok = false; break; }
+                        if (!wait_pv_done(X, t - 1, kPPvDone)) { ok = false; break; }
                         pv_waited = true;
                     }
                     tc_fence_after();
@@ -601,7 +601,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                     if (c == kFirstStoreChunk && !pv_waited) {
                         // P has its own columns: the P V that read the previous P must be done before
                         // they change.  The first chunks of P stay in registers meanwhile.
-                        if (!__all_sync(0xffffffffu, wait_pv_done(X, t - 1, kPPvDone))) { ok = false; break; }
+                        if (!wait_pv_done(X, t - 1, kPPvDone)) { ok = false; break; }
                         tc_fence_after();
                         pv_waited = true;
                     }
@@ -632,7 +632,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (lse_out != nullptr && row < seq_len)
                 lse_out[static_cast<size_t>(it.bh) * seq_len + row] = kLn2 * (m_run + log2f(l_run));
             if (itx > 0 &&
-                !__all_sync(0xffffffffu, mbar_wait(smem_u32(&cb.stats_free[X]), (itx - 1) & 1, ctl, kPStatsFree))) break;
+                !mbar_wait(smem_u32(&cb.stats_free[X]), (itx - 1) & 1, ctl, kPStatsFree)) break;
             cb.inv_l[X][r_in_tile] = 1.0f / l_run;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&cb.stats_full[X]));

@@ -102,14 +102,12 @@ struct WaitCtl {
     int*          status;       // in global memory: first error word of the launch wins
 };
 
-// Waits for the phase with the given parity to complete.  Returns false if the
-// CTA is aborting (this waiter timed out, or another one did).  The loop itself is
-// bounded_wait() (bounded_wait.h), which a host test drives through its give-up branch.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtl& ctl,
-                                          int barrier_id) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const int r = bounded_wait([&] { return mbar_try_wait_parked(bar, parity, kParkNs); },
-                               [&] { return *ctl.abort_flag != 0; }, [] { return global_timer_ns(); },
+// One lane's bounded wait for what `try_wait` asks for.  Returns false if the CTA is aborting (this lane timed
+// out, or another waiter did).  The loop itself is bounded_wait() (bounded_wait.h), which a host test drives
+// through its give-up branch.
+template <class TryWait>
+__device__ __forceinline__ bool lane_wait(TryWait try_wait, const WaitCtl& ctl, int barrier_id) {
+    const int r = bounded_wait(try_wait, [&] { return *ctl.abort_flag != 0; }, [] { return global_timer_ns(); },
                                kWaitLimitNs, 16u);
     if (r == kWaitDone) return true;
     if (r == kWaitTimedOut) {
@@ -117,6 +115,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const W
         atomicCAS(ctl.status, 0, wait_timeout_word(barrier_id));
     }
     return false;
+}
+__device__ __forceinline__ bool warp_all(bool x) { return __all_sync(0xffffffffu, x) != 0; }
+
+// Waits for the phase with the given parity to complete: executed by a whole warp, either with the same answer
+// in every lane (false if the CTA is aborting), or noting it in `lw` for the vote after an issue.
+__device__ __forceinline__ bool lane_mbar_wait(uint32_t bar, uint32_t parity, const WaitCtl& ctl, int barrier_id) {
+    return mbar_try_wait(bar, parity) || lane_wait([&] { return mbar_try_wait_parked(bar, parity, kParkNs); }, ctl, barrier_id);
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtl& ctl, int barrier_id) {
+    return warp_wait([&] { return lane_mbar_wait(bar, parity, ctl, barrier_id); }, warp_all);
+}
+__device__ __forceinline__ void mbar_wait(LaneWaits& lw, uint32_t bar, uint32_t parity, const WaitCtl& ctl, int barrier_id) {
+    lw.wait([&] { return lane_mbar_wait(bar, parity, ctl, barrier_id); });
 }
 
 // ---------------------------------------------------------------------------
@@ -368,17 +379,9 @@ __device__ __forceinline__ bool mbar_try_wait_parked_cluster(uint32_t bar, uint3
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const WaitCtl& ctl,
+__device__ __forceinline__ void mbar_wait_cluster(LaneWaits& lw, uint32_t bar, uint32_t parity, const WaitCtl& ctl,
                                                   int barrier_id) {
-    const int r = bounded_wait([&] { return mbar_try_wait_parked_cluster(bar, parity, kParkNs); },
-                               [&] { return *ctl.abort_flag != 0; }, [] { return global_timer_ns(); },
-                               kWaitLimitNs, 16u);
-    if (r == kWaitDone) return true;
-    if (r == kWaitTimedOut) {
-        *ctl.abort_flag = 1;
-        atomicCAS(ctl.status, 0, wait_timeout_word(barrier_id));
-    }
-    return false;
+    lw.wait([&] { return lane_wait([&] { return mbar_try_wait_parked_cluster(bar, parity, kParkNs); }, ctl, barrier_id); });
 }
 // Whole-warp calls, executed by the same warp index in BOTH CTAs of the pair with the same slot address.
 __device__ __forceinline__ void tmem_alloc_2sm(uint32_t smem_slot, uint32_t ncols) {

@@ -57,6 +57,7 @@
 
 #include "fast_div.h"
 #include "host_common.h"
+#include "page_entry.h"
 #include "ptx.cuh"
 #include "tmem_ld.cuh"
 
@@ -338,9 +339,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // now 40.2).  The producers have a loop for either kind of cache: a few more instructions
     // per tile on the other one cost D=128 chunks 3-5 %.
     auto cache_pages = [&](const Item& it, int j) -> int {
-        const int off = lane << gq.page_shift, rr = (it.t0 + j) * kBN + off;
-        if (off >= kBN || rr >= it.kv_len || j >= it.n_kv) return -1;
-        return gq.block_table[static_cast<size_t>(it.b) * gq.table_stride + (rr >> gq.page_shift)];
+        const int e = page_entry(lane, (it.t0 + j) * kBN, it.kv_len, gq.page_shift);
+        if (e < 0 || j >= it.n_kv) return -1;
+        return gq.block_table[static_cast<size_t>(it.b) * gq.table_stride + e];
     };
     auto load_cache_tile = [&](uint32_t dst, uint32_t bytes, const CUtensorMap* tm, uint32_t bar, const Item& it, int j, int pages, auto paged) {
         constexpr int NB = FP8 ? 1 : NBOX;            // boxes per tile row: e4m3 rows are one 128-byte box

@@ -300,7 +300,8 @@ decode_cluster_kernel(const uint16_t* q, const uint16_t* k, const uint16_t* v,
 // ([rank][row][D + 1], LSE in the last column), and can write a packed row itself.
 // The parts are dealt to the warps, a lane taking every 32nd element of each (d_head 64: the second 64 of
 // the 128 accumulator slots stay empty); a thread that walks all parts of its element alone waits for one
-// pair of dependent loads after the other (B*H=8 Skv=131072, 148 splits, whole call: 93 us, now 85).
+// pair of dependent loads after the other (B*H=8 Skv=131072, 148 splits, whole call: 93 us, now 85).  For many
+// parts and few rows.
 constexpr int kCombineMaxWarps = 8;
 template <bool BF16>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32)
@@ -344,6 +345,34 @@ combine_kernel(const float* o_parts, const float* lse_parts,
     }
 }
 
+// The same merge with one thread per head-dim element, which walks all parts: no shared memory and no barrier
+// (combine_by_warps says where which one runs).
+template <bool BF16>
+__global__ void combine_rows_kernel(const float* o_parts, const float* lse_parts,
+                                    int n_parts, long long part_stride_o, long long row_stride_o,
+                                    long long part_stride_l, long long row_stride_l, int d_head,
+                                    uint16_t* o, float* lse, long long lse_stride,
+                                    float* o_f32, long long o_f32_stride) {
+    const int row = blockIdx.x, d = threadIdx.x;
+    grid_dependency_wait();
+    // no grid_launch_dependents: with many CTAs the instruction itself costs (65536 rows of 1 part, 1 CTA a row: 37 us
+    // without, 69 with), and a dependent that starts when this grid completes loses nothing measurable
+    const float* lp = lse_parts + (size_t)row * row_stride_l;
+    float m = -INFINITY;
+    for (int p = 0; p < n_parts; p++) m = fmaxf(m, lp[(size_t)p * part_stride_l]);
+    float wsum = 0.0f, a = 0.0f;
+    if (m > -INFINITY) {
+        const float* op = o_parts + (size_t)row * row_stride_o + d;
+        for (int p = 0; p < n_parts; p++) {
+            const float w = fast_ex2((lp[(size_t)p * part_stride_l] - m) * kLog2e);
+            wsum += w;
+            a = fmaf(w, op[(size_t)p * part_stride_o], a);
+        }
+    }
+    write_row<BF16>(row, d, d_head, wsum > 0.0f ? a / wsum : 0.0f, wsum > 0.0f ? m + kLn2 * log2f(wsum) : -INFINITY, o, lse, lse_stride,
+                    o_f32, o_f32_stride);
+}
+
 // A rank that holds no key of a KV-sequence-sharded cache contributes weight zero to the merge.
 __global__ void empty_partial_kernel(float* packed, int d_head) {
     float* row = packed + (size_t)blockIdx.x * (d_head + 1);
@@ -359,14 +388,26 @@ struct CombineOut {
     long long o_f32_stride = 0;
 };
 
+// Which merge kernel.  Dealing the parts to warps shortens a row's chain of dependent loads, but every warp reads
+// the row's LSEs and the warps meet at a barrier: it pays where a row has many parts and the GPU few rows; many
+// rows hide the chain by themselves.  Whole call on cold inputs (one thread an element / by warps, us), d_head 64:
+// 16 parts: 444 rows 10.3 / 9.1, 1184 rows 10.3 / 12.4, 4096 rows 12.4 / 22.5, 32768 rows 46 / 119; 64 parts: 888 rows
+// 20.5 / 14.4, 1184 rows 20.9 / 20.5, 2368 rows 22.5 / 28.7; 8 parts: 296 rows 8.2 / 8.2 (in a graph, inputs in L2,
+// 1.9 / 2.1), 4096 rows 10.3 / 14.4.  In a graph 16 parts of 592 rows take 2.5 / 3.3, 148 parts 11.2 / 9.9.
+bool combine_by_warps(int n_parts, int rows, int sm_count) {
+    return n_parts > 8 && rows <= (n_parts >= 64 ? 6 : 3) * sm_count;
+}
+
 int launch_combine(const float* o_parts, const float* lse_parts, int n_parts, long long pso,
                    long long rso, long long psl, long long rsl, int rows, int d_head, const CombineOut& out,
-                   int dtype, cudaStream_t stream) {
-    // two parts a warp, so that a warp's loads are in flight together and few warps idle
+                   int dtype, int sm_count, cudaStream_t stream) {
+    const bool bf = dtype == FA_DTYPE_BF16;
+    const bool by_warps = combine_by_warps(n_parts, rows, sm_count);
+    auto kernel = by_warps ? (bf ? combine_kernel<true> : combine_kernel<false>) : (bf ? combine_rows_kernel<true> : combine_rows_kernel<false>);
+    // by warps: two parts a warp, so that a warp's loads are in flight together and few warps idle
     const int warps = n_parts >= 2 * kCombineMaxWarps ? kCombineMaxWarps : (n_parts + 1) / 2;
-    return launch_dependent(dtype == FA_DTYPE_BF16 ? combine_kernel<true> : combine_kernel<false>, rows, warps * 32, 0, stream, 1, o_parts,
-                            lse_parts, n_parts, pso, rso, psl, rsl, d_head, static_cast<uint16_t*>(out.o), out.lse, out.lse_stride,
-                            out.o_f32, out.o_f32_stride);
+    return launch_dependent(kernel, rows, by_warps ? warps * 32 : d_head, 0, stream, 1, o_parts, lse_parts, n_parts, pso, rso, psl, rsl, d_head,
+                            static_cast<uint16_t*>(out.o), out.lse, out.lse_stride, out.o_f32, out.o_f32_stride);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -463,7 +504,7 @@ int decode_into(const fa_decode_args* a, int splits, int kps, int sm_count, void
     if (rc != FA_OK) return rc;
     // partials: o [bh][split][D], lse [bh][split]
     return launch_combine(o_part, lse_part, splits, a->d_head, (long long)splits * a->d_head, 1, splits,
-                          (int)bh, a->d_head, out, a->dtype, stream);
+                          (int)bh, a->d_head, out, a->dtype, sm_count, stream);
 }
 
 CombineOut caller_outputs(const fa_decode_args* a) {
@@ -685,7 +726,7 @@ FA_EXPORT int fa_decode_gqa(const fa_decode_gqa_args* a) {
     CombineOut out;
     out.o = a->o; out.lse = a->lse;
     return launch_combine(o_part, lse_part, splits, a->d_head, (long long)splits * a->d_head, 1, splits,
-                          (int)rows, a->d_head, out, e4m3 ? FA_DTYPE_BF16 : a->dtype, stream);
+                          (int)rows, a->d_head, out, e4m3 ? FA_DTYPE_BF16 : a->dtype, st->sm_count, stream);
 }
 
 FA_EXPORT int fa_combine(const float* o_parts, const float* lse_parts, int n_parts, int rows,
@@ -699,7 +740,7 @@ FA_EXPORT int fa_combine(const float* o_parts, const float* lse_parts, int n_par
     CombineOut out;
     out.o = o; out.lse = lse;
     return launch_combine(o_parts, lse_parts, n_parts, (long long)rows * d_head, d_head, rows, 1, rows,
-                          d_head, out, dtype, static_cast<cudaStream_t>(stream));
+                          d_head, out, dtype, st->sm_count, static_cast<cudaStream_t>(stream));
 }
 
 FA_EXPORT int fa_combine_packed(const float* packed_parts, int n_parts, int rows, int d_head, void* o,
@@ -714,7 +755,7 @@ FA_EXPORT int fa_combine_packed(const float* packed_parts, int n_parts, int rows
     CombineOut out;
     out.o = o; out.lse = lse;
     return launch_combine(packed_parts, packed_parts + d_head, n_parts, (long long)rows * w, w, (long long)rows * w, w,
-                          rows, d_head, out, dtype, static_cast<cudaStream_t>(stream));
+                          rows, d_head, out, dtype, st->sm_count, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------

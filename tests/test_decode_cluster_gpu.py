@@ -46,7 +46,19 @@ def test_decode_shapes(fa, dev, oracle, bh, kv, splits, d, dtype):
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("packed", [False, True])
 def test_combine_part_counts(fa, dev, n_parts, d, packed):
-    rows = 7
+    check_combine(fa, dev, n_parts, 7, d, packed)
+
+
+@pytest.mark.parametrize("n_parts,rows_per_sm", [(8, 3), (9, 3), (63, 3), (63, 6), (64, 3), (64, 6)])
+@pytest.mark.parametrize("beyond", [0, 1])
+@pytest.mark.parametrize("d,packed", [(64, True), (128, False)])
+def test_combine_row_counts(fa, dev, n_parts, rows_per_sm, beyond, d, packed):
+    """Both merge kernels on both sides of the line between them."""
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    check_combine(fa, dev, n_parts, rows_per_sm * sms + beyond, d, packed)
+
+
+def check_combine(fa, dev, n_parts, rows, d, packed):
     gen = torch.Generator(device=dev).manual_seed(n_parts * d)
     o = torch.randn((n_parts, rows, d), generator=gen, device=dev)
     lse = torch.randn((n_parts, rows), generator=gen, device=dev) * 4

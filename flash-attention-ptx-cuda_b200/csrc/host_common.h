@@ -74,8 +74,10 @@ inline int launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block,
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    FA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
-    return FA_OK;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (err == cudaSuccess) return FA_OK;
+    cudaGetLastError();                  // reported here: the caller's next check must not find it
+    return note_cuda_error(err, "cudaLaunchKernelEx");
 }
 
 // Rank-3 tiled tensor map over a dense [n_heads, n_rows, row_elems] tensor with

@@ -56,7 +56,9 @@ int note_message(const char* msg, int code);
 
 // Launches `kernel` as a programmatic dependent of whatever precedes it on the stream (cluster of
 // `cluster` CTAs): its launch and set-up overlap the end of that work.  The kernel must execute
-// grid_dependency_wait() before its first access to global memory.
+// grid_dependency_wait() before its first access to global memory, and signal (grid_launch_dependents) only
+// after that wait, so that a kernel whose predecessor has signalled knows all work before the predecessor to be
+// complete.  One kernel relies on that instead of waiting itself: the dQ kernel of the backward (backward.cu).
 template <class... P, class... A>
 inline int launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, unsigned cluster,
                             const A&... args) {

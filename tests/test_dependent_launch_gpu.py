@@ -118,3 +118,44 @@ def test_captured_after_a_copy_and_a_join(fa, dev):
         torch.cuda.synchronize()
         assert torch.equal(q, ref[0]) and torch.equal(lse, ref[1])
     assert fa.device_status() == 0
+
+
+@pytest.mark.parametrize("d,dtype", [(64, "f16"), (128, "bf16")])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("b,h,s", [(1, 3, 130), (2, 40, 300), (1, 5, 1100)])
+def test_backward_calls_in_a_row(fa, dev, d, dtype, causal, b, h, s):
+    """Calls on changing data with one workspace: the dQ kernel starts before the dK/dV kernel has ended and reads
+    the delta that this call's first kernel has just written over the last call's."""
+    gen = torch.Generator(device=dev).manual_seed(s + d)
+    t = torch.float16 if dtype == "f16" else torch.bfloat16
+    scale = d ** -0.5
+    sets = []
+    for i in range(3):
+        q, k, v, d_o = (rnd(gen, dev, b, h, s, d, dtype=t) * (1 + i) for _ in range(4))
+        o, lse = torch.empty_like(q), torch.empty((b, h, s), device=dev)
+        fa.prefill(q, k, v, o, lse, b, h, s, d, scale, causal, dtype=dtype)
+        sets.append((q, k, v, o, d_o, lse))
+    ws = torch.zeros(fa.backward_workspace_bytes(b, h, s), device=dev, dtype=torch.uint8)
+
+    def run(sync):
+        outs = []
+        for i in range(12):
+            x = sets[i % 3]
+            outs.append([torch.full_like(x[0], float("nan")) for _ in range(3)])
+            torch.cuda.synchronize()
+        for i, out in enumerate(outs):
+            fa.backward(*sets[i % 3], *out, b, h, s, d, scale, causal, dtype=dtype, workspace=ws, workspace_bytes=ws.numel(),
+                        stream=torch.cuda.current_stream(dev))
+            if sync:
+                torch.cuda.synchronize()
+                ws.fill_(255)                              # a delta read too early would be a NaN
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    ref = run(True)
+    assert all(torch.isfinite(x.float()).all() for out in ref for x in out)
+    for _ in range(3):
+        for x, y in zip(run(False), ref):
+            assert all(torch.equal(a, c) for a, c in zip(x, y))
+    assert fa.device_status() == 0

@@ -657,10 +657,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // ---- e4m3 -> fp16 conversion of the item's V tiles (exact)
                 for (int j = 0; j < it.n_kv; j++, g++) {
                     const int s8 = g % L::NV8, sv = g % NV;
-                    bool w = mbar_wait(smem_u32(&bar_v8f[s8]), (g / L::NV8) & 1, ctl, kBarV8Full);
+                    LaneWaits lw;
+                    mbar_wait(lw, smem_u32(&bar_v8f[s8]), (g / L::NV8) & 1, ctl, kBarV8Full);
                     // the fp16 buffer must have been consumed by the P V that last read it
-                    if (g >= NV) w = w && mbar_wait(smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty);
-                    if (!w) { ok = false; break; }
+                    if (g >= NV) mbar_wait(lw, smem_u32(&bar_pvd[(g - NV) % kRing]), ((g - NV) / kRing) & 1, ctl, kBarVEmpty);
+                    if (!warp_all(lw.ok)) { ok = false; break; }
                     const uint32_t src_base = v8_s + s8 * L::kV8Bytes;
                     const uint32_t dst_base = v_s + sv * L::kVBytes;
                     // decode over a cache: rows past the sequence's end may hold stale bytes (NaN codes
@@ -727,10 +728,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // an item of a single tile has used one accumulator only
                 const bool has_b = it.n_kv > 1;
                 g += it.n_kv;
-                bool w = mbar_wait(smem_u32(&bar_odone[ga]), (used >> ga) & 1, ctl, kBarODone);
-                if (has_b) w = w && mbar_wait(smem_u32(&bar_odone[ga ^ 1]), (used >> (ga ^ 1)) & 1, ctl, kBarODone);
+                LaneWaits lw;
+                mbar_wait(lw, smem_u32(&bar_odone[ga]), (used >> ga) & 1, ctl, kBarODone);
+                if (has_b) mbar_wait(lw, smem_u32(&bar_odone[ga ^ 1]), (used >> (ga ^ 1)) & 1, ctl, kBarODone);
                 used ^= has_b ? 3u : 1u << ga;
-                if (!w) break;
+                if (!warp_all(lw.ok)) break;
                 tc_fence_after();
                 // the staging buffer must have been drained by the previous item's TMA store
                 if (tid == 384) tma_store_wait_read();

@@ -27,7 +27,7 @@ def test_give_up_branch_on_the_host(tmp_path):
 
 def test_no_kernel_leaves_a_loop_lane_by_lane():
     """Outside of ptx.cuh a kernel uses the voting waits, votes on ``bounded_wait`` itself, or votes on the
-    ``LaneWaits`` of an issue right after it."""
+    ``LaneWaits`` that an issue or several waits share."""
     for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         with open(path) as f:
             text = f.read()

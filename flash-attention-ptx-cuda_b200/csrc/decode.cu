@@ -390,13 +390,12 @@ struct CombineOut {
 
 // Which merge kernel.  Dealing the parts to warps shortens a row's chain of dependent loads, but every warp reads
 // the row's LSEs and the warps meet at a barrier: it pays where a row has many parts and the GPU few rows; many
-// rows hide the chain by themselves.  Whole call on cold inputs (one thread an element / by warps, us), d_head 64:
-// 16 parts: 444 rows 10.3 / 9.1, 1184 rows 10.3 / 12.4, 4096 rows 12.4 / 22.5, 32768 rows 46 / 119; 64 parts: 888 rows
-// 20.5 / 14.4, 1184 rows 20.9 / 20.5, 2368 rows 22.5 / 28.7; 8 parts: 296 rows 8.2 / 8.2 (in a graph, inputs in L2,
-// 1.9 / 2.1), 4096 rows 10.3 / 14.4.  In a graph 16 parts of 592 rows take 2.5 / 3.3, 148 parts 11.2 / 9.9.
-bool combine_by_warps(int n_parts, int rows, int sm_count) {
-    return n_parts > 8 && rows <= (n_parts >= 64 ? 6 : 3) * sm_count;
-}
+// rows hide the chain by themselves.  One thread an element / by warps, us, whole call on cold inputs, d_head 64:
+// 16 parts: 444 rows 10.3 / 9.1, 888 rows 10.6 / 10.2, 1184 rows 10.3 / 12.4, 4096 rows 12.4 / 22.5, 32768 rows
+// 46 / 119; 64 parts: 888 rows 20.5 / 14.4, 1184 rows 20.9 / 20.5, 2368 rows 22.5 / 28.7; 8 parts: 296 rows 8.2 /
+// 8.2 (in a graph, inputs in L2, 1.9 / 2.1), 4096 rows 10.3 / 14.4.  After the partials' kernel, calls in a row:
+// 9 parts of 1024 rows (B=32 Hq=32 Hkv=1 Skv=32768 D=128) 95.5 / 93.2.
+bool combine_by_warps(int n_parts, int rows, int sm_count) { return n_parts > 8 && rows <= 7ll * sm_count; }
 
 int launch_combine(const float* o_parts, const float* lse_parts, int n_parts, long long pso,
                    long long rso, long long psl, long long rsl, int rows, int d_head, const CombineOut& out,

@@ -49,7 +49,7 @@ def test_combine_part_counts(fa, dev, n_parts, d, packed):
     check_combine(fa, dev, n_parts, 7, d, packed)
 
 
-@pytest.mark.parametrize("n_parts,rows_per_sm", [(8, 3), (9, 3), (63, 3), (63, 6), (64, 3), (64, 6)])
+@pytest.mark.parametrize("n_parts,rows_per_sm", [(8, 3), (8, 7), (9, 7), (64, 7)])
 @pytest.mark.parametrize("beyond", [0, 1])
 @pytest.mark.parametrize("d,packed", [(64, True), (128, False)])
 def test_combine_row_counts(fa, dev, n_parts, rows_per_sm, beyond, d, packed):

@@ -58,6 +58,8 @@
 // S=4096 531 instead of 471.  The per-step waits of a compute warp (products ready, operand columns
 // free, stores complete) are latencies that only other warps' work can fill, hence sixteen compute
 // warps on two steps rather than eight on one.
+// Times in these comments are of calls in a row on the same buffers, each pair from one box and the build in
+// which that step was made.
 #include <cmath>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -330,7 +332,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 }
                 tc_fence_after();
                 const uint64_t db0 = make_sdesc(b_s + s * 2 * L::kTileB, hi_k), db1 = db0 + (L::kTileB >> 4);
-                if (elect_one() && lw.ok) {
+                if (!warp_all(lw.ok)) { ok = false; break; }
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
@@ -344,7 +347,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     if (T >= 2) mbar_wait(lw, smem_u32(&bar_acc1[(T - 2) % kStages]), ((T - 2) / kStages) & 1, ctl, kBwdBarAcc);
                     tc_fence_after();
                 }
-                if (elect_one() && lw.ok) {
+                if (!warp_all(lw.ok)) { ok = false; break; }
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < D / 16; kk++) {
                         const uint32_t offa = ((kk >> 2) * L::kBox + (kk & 3) * 32) >> 4, offb = ((kk >> 2) * L::kBoxB + (kk & 3) * 32) >> 4;
@@ -352,7 +356,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                     }
                     tc_commit(smem_u32(INPLACE ? &bar_t1[g] : &bar_t[g]));
                 }
-                if (!warp_all(lw.ok)) { ok = false; break; }
+                __syncwarp();
                 issued = true;
             }
             if (!ok) break;
@@ -387,14 +391,15 @@ bwd_kernel(const __grid_constant__ CUtensorMap ta0, const __grid_constant__ CUte
                 tc_fence_after();
                 const uint64_t db = make_sdesc(b_s + s * 2 * L::kTileB + (use_p ? L::kTileB : 0), hi_mn);
                 const uint32_t op = op0 + g * OP_STRIDE;
-                if (elect_one() && lw.ok) {
+                if (!warp_all(lw.ok)) { ok = false; break; }
+                if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < kW / 16; kk++)
                         mma_f16_ts(acc, op + op16_col(kk, INPLACE), db + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
                     tc_commit(smem_u32(INPLACE && x == 1 ? &bar_acc1[s] : &bar_acc[s]));
                     if (t == it.n_steps - 1) tc_commit(smem_u32(&bar_done));
                 }
-                if (!warp_all(lw.ok)) { ok = false; break; }
+                __syncwarp();
             }
             gs += it.n_steps;
         }

@@ -345,6 +345,7 @@ combine_kernel(const float* o_parts, const float* lse_parts,
     }
 }
 
+constexpr unsigned kSignalRows = 1024;
 // The same merge with one thread per head-dim element, which walks all parts: no shared memory and no barrier
 // (combine_by_warps says where which one runs).
 template <bool BF16>
@@ -355,8 +356,10 @@ __global__ void combine_rows_kernel(const float* o_parts, const float* lse_parts
                                     float* o_f32, long long o_f32_stride) {
     const int row = blockIdx.x, d = threadIdx.x;
     grid_dependency_wait();
-    // no grid_launch_dependents: with many CTAs the instruction itself costs (65536 rows of 1 part, 1 CTA a row: 37 us
-    // without, 69 with), and a dependent that starts when this grid completes loses nothing measurable
+    // With many CTAs the signal itself costs, ~0.5 ns a CTA (65536 rows of 1 part: 37 us without, 69 with); with few the
+    // next kernel's set-up that it lets overlap is worth more (grouped-query decode, B=2 Hq=32 Hkv=8 Skv=2048, calls in a
+    // row: 11.4 us with, 12.0 without).
+    if (gridDim.x <= kSignalRows) grid_launch_dependents();
     const float* lp = lse_parts + (size_t)row * row_stride_l;
     float m = -INFINITY;
     for (int p = 0; p < n_parts; p++) m = fmaxf(m, lp[(size_t)p * part_stride_l]);
@@ -453,7 +456,7 @@ void plan_splits(const fa_decode_args* a, int sm_count, int* splits_out, int* ke
 // CTAs per head of the one-launch path, 0 = take the two-launch path.  A head's splits must fit the portable
 // cluster size, and the whole grid the GPU at once (four CTAs of 8 warps an SM): a cluster keeps its
 // CTAs until the last has finished, so with more than one wave of them the two launches are as fast or
-// faster (f16 D=64 B*H=1024 Skv=4096, 4 splits: 180 against 159 us; bf16 D=128 B*H=128 Skv=4096, 8 splits: 49.3
+// faster (calls in a row, f16 D=64 B*H=1024 Skv=4096, 4 splits: 180 against 159 us; bf16 D=128 B*H=128 Skv=4096, 8 splits: 49.3
 // against 47.9; bf16 D=64 B*H=128 Skv=2048, 4 splits, 512 CTAs: 14.4 against 15.2).  Heads that leave the GPU
 // empty get more CTAs than splits, up to two a SM and down to 64 keys each.
 int decode_cluster_ctas(long long bh, int splits, int seq_len_kv, int sm_count) {

@@ -15,11 +15,11 @@
 //     split): a normalised fp32 partial O and its natural-log LSE.
 //   decode_cluster_kernel  the same pass when a head needs at most 8 CTAs: they form a thread-block
 //     cluster and merge through distributed shared memory, so that one launch writes the result.
-//   combine_kernel  merges partials by their LSEs,
+//   combine_kernel, combine_rows_kernel  merge partials by their LSEs,
 //       m = max lse_p, w_p = exp(lse_p - m), O = sum w_p O_p / sum w_p,
 //       LSE = m + log(sum w_p),
-//     converts to the 16-bit output type, and can also emit the fp32 result.
-//     The same kernel merges the per-GPU partials of KV-sequence-sharded decode
+//     convert to the 16-bit output type, and can also emit the fp32 result.
+//     They also merge the per-GPU partials of KV-sequence-sharded decode
 //     (parts = ranks), reading the gathered buffer directly.
 #include <cfloat>
 #include <cmath>

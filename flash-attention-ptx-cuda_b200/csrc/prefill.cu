@@ -51,6 +51,10 @@
 //
 // TMEM (all 512 columns): three score buffers [0,128) [128,256) [256,384), O [384,384+D)
 // (SPLIT: two accumulators, [384,448) and [448,512)).
+//
+// Times in the comments below are of calls in a row on the same buffers (inputs up to the size of L2 are warm
+// then, and a call's launch overlaps the end of the one before), each pair from one box and the build
+// in which that step was made: they compare within a pair, and are below what a lone call takes.
 #include <atomic>
 #include <cmath>
 #include <type_traits>
@@ -106,10 +110,11 @@ struct PrefillSmem {
     static constexpr int kVBytes  = kNBox * kBox;         // 16-bit V operand of P V (e4m3: converted copy)
     static constexpr int kV8Bytes = V8 ? kBox : 0;       // landing buffers of the e4m3 V tiles
     static constexpr int kOBytes  = SMALL ? 0 : kNBox * kBox;   // epilogue staging (16-bit output tile)
-    // V8 (decode over an e4m3 cache): three landing buffers of K and V and two converted (fp16) V tiles; the bytes in
-    // flight are what the cache's bandwidth needs (2, 2 and 3, the same shared memory: 198 us instead of 181,
-    // B=32 Hkv=8 Skv=16384).  SMALL has no output to stage and takes the room for loads in flight as well: with
-    // two stages a lone CTA waits for a load's latency every other tile (see `ahead` at the launch).
+    // V8 (decode over an e4m3 cache): three landing buffers of K and of V and two converted (fp16) V tiles; the bytes
+    // in flight are what the cache's bandwidth needs (2, 2 and 3, the same shared memory: 198 us instead of 181,
+    // B=32 Hkv=8 Skv=16384).  SMALL has no output to stage and takes that room for loads in flight as well: four
+    // landing buffers of each (V8), three stages instead of two (D 128), six instead of four (D 64); how many
+    // of a 16-bit cache's stages are used is decided at the launch (`ahead`).
     static constexpr int NK  = (D == 64) ? (SMALL ? 6 : 4) : V8 ? (SMALL ? 4 : 3) : (SMALL ? 3 : 2);
     static constexpr int NV  = (D == 64) ? (SMALL ? 6 : 4) : V8 ? 2 : (SMALL ? 3 : 2);
     static constexpr int NV8 = V8 ? (SMALL ? 4 : 3) : 0;
@@ -669,10 +674,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     const int valid = GQA ? it.kv_len - (it.t0 + j) * kBN : kBN;
                     // A thread takes 16 codes (one 16-byte chunk) of eight rows, all loaded before the first is
                     // used: 8 bytes at a time, a few in flight, the loads' latency made this the slowest role
-                    // of the kernel (B=32 Hkv=8 Skv=16384: 258 us, now 225, and 213 with the loads above changed too).  Codes 16 ch .. 16 ch + 15 become the chunks
-                    // 2 ch and 2 ch + 1 of a 256-byte fp16 row (two boxes of 8 chunks); the threads of the
-                    // second box write their odd chunk first, so that a quarter warp, which covers one row,
-                    // meets every bank once.
+                    // of the kernel (B=32 Hkv=8 Skv=16384: 258 us, now 225).  Codes 16 ch .. 16 ch + 15 become
+                    // the chunks 2 ch and 2 ch + 1 of a 256-byte fp16 row (two boxes of 8 chunks); the threads
+                    // of the second box write their odd chunk first, so that a quarter warp, which covers one
+                    // row, meets every bank once.
                     const int ch = ct & 7, r0 = ct >> 3;             // chunk; first row (then every 16th)
                     uint4 c[8];
 #pragma unroll
@@ -1302,9 +1307,13 @@ int launch_gqa_instance(const GqaLaunch& g, DeviceState* st, const CUtensorMap& 
     // tile reads everything once, in any order.
     const int walk = n_qt > 1 ? heads_per_group(n_bh, g.kv_len, g.d_head, FP8 ? 1 : 2) : n_bh;
     // SMALL, 16-bit cache: how many of the stages to use.  All of them where CTAs are left alone with long
-    // sequences while the rest have finished (lengths differ, at most two items a CTA): one CTA then gets
-    // more of the bandwidth (B=16 Hkv=8 Skv<=4096 D=128 paged 37.5 -> 32.9 us, not paged 34.2 -> 32.3).  When
-    // every SM streams to the end the deeper queues cost DRAM efficiency (B=32 Hkv=8 Skv=16384 312 -> 326).
+    // sequences while the rest have finished: one CTA then gets more of the bandwidth (d_head 128, lengths from
+    // 1/16 of Skv up, cold inputs, two thirds / all of the stages: B=16 Hkv=8 Skv=4096 paged 48.1 / 43.9 us, B=32 Hkv=1
+    // Skv=16384 paged 50.2 / 44.0).  When every SM streams to the end the deeper queues cost DRAM efficiency
+    // (B=32 Hkv=8 Skv=16384 equal lengths, calls in a row: 309 / 329).  The host does not know the lengths: the rule takes
+    // `seq_lens` given and at most two items a CTA for the first situation.  So equal lengths passed in
+    // `seq_lens` get all stages too, up to 4 % slower (B=16 Hkv=8 Skv=4096 44.6 / 46.2), and d_head 64, whose six
+    // stages gain nothing with different lengths (19.8 / 19.8), loses up to 5 % with equal ones (26.1 / 27.3).
     const int ahead = g.seq_lens != nullptr && n_items <= 2ll * st->sm_count ? L::NK : L::NK / 3 * 2;
     const int last_heads = n_bh % walk ? n_bh % walk : walk;
     const GqaDev gq{g.o_part, g.lse_part, static_cast<uint16_t*>(g.o_final), g.lse_final, g.n_splits,

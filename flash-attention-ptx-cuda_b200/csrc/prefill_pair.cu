@@ -22,7 +22,7 @@
 //                     exceeds it by more than 2^8.
 //   warp 8            TMA producer: Q of both tiles per item, the K ring.
 //   warp 11           TMA producer: the V ring (a V slot frees much later than a K slot).
-//   warp 9 / warp 10  MMA issuer of tile A / tile B (lane 0 issues): S = Q K^T into the
+//   warp 9 / warp 10  MMA issuer of tile A / tile B (an elected lane): S = Q K^T into the
 //                     tile's score buffer, O += P V with P from TMEM and V (MN-major) from
 //                     shared memory.  Instructions of one thread execute in order, which is
 //                     what lets P alias S at d_head 128.

@@ -118,7 +118,10 @@ int fa_prefill_host(const fa_prefill_args* args_with_host_pointers);
  *
  * The key range is cut into num_splits contiguous slices (0 = choose); each
  * slice produces a partial (O, LSE) in `workspace`, and a second kernel merges
- * the partials by their LSEs and writes o (16-bit) and, if given, lse.
+ * the partials by their LSEs and writes o (16-bit) and, if given, lse.  A short
+ * job (at most 8 slices, all of them on the GPU at once) is done by one kernel
+ * instead: it may cut the keys into more slices than num_splits and leaves the
+ * workspace untouched.  Its size is checked either way.
  * If o_f32 is non-NULL the merged, normalised output is ALSO written there in
  * fp32 ([batch_size*num_heads, d_head]); together with lse this is the partial
  * result a rank contributes when the KV sequence is sharded across GPUs.
